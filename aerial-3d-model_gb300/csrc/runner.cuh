@@ -481,8 +481,13 @@ struct LmEngine {
   detail::PcgPlan plan;
   DevBuf<PcgJob> jobs;
   DevBuf<int32_t> cta_job0;
-  DevBuf<unsigned long long> bar, bar_base;
+  DevBuf<unsigned long long> bar, bar_base;  // matrix-free kernel
   DevBuf<double> pcg_part;
+  // Grid kernel: sequence numbers, exchange words (partial sums, z) and the
+  // previous p of blocks that shared memory does not hold.
+  DevBuf<unsigned long long> pcg_epoch;
+  DevBuf<PcgWord> pcg_words, pcg_said, pcg_zx;
+  DevBuf<R> pblk;
   DevBuf<int32_t> lens_row, lens_pos;
   uint32_t smem_rows = 0, smem_blocks = 0;
   uint32_t sub_len = kSubLen;  // Schur pairs per warp sub-segment
@@ -667,7 +672,6 @@ struct LmEngine {
     }
     pre.alloc(at_least_1(nb) * 36, s);
     g.alloc(at_least_1(nb) * 6, s), x.alloc(at_least_1(nb) * 6, s);
-    z.alloc(at_least_1(nb) * 6, s), p.alloc(at_least_1(nb) * 12, s);
     cost_part.alloc(at_least_1(SB.ncost) * 3, s);
     // Camera sums are read for every camera, including ones without observations.
     camU.zero(), camgj.zero(), camgs.zero(), camX.zero(), caml.zero(), grpU.zero(), grpg.zero();
@@ -739,7 +743,8 @@ struct LmEngine {
     const int64_t rows_fit = (int64_t)(kPcgSmemBudget / row_bytes);
     const int64_t rows_need = (nb * 5 / 4 + max_ctas - 1) / max_ctas + 8;
     smem_rows = (uint32_t)std::min<int64_t>(rows_fit, std::max<int64_t>(64, rows_need));
-    smem_blocks = (uint32_t)((kPcgSmemBudget - (size_t)smem_rows * row_bytes) / (36 * sizeof(R) + 4));
+    smem_blocks =
+        (uint32_t)((kPcgSmemBudget - (size_t)smem_rows * row_bytes) / pcg_block_bytes<R>());
     smem_bytes = pcg_smem_bytes<R>(smem_rows, smem_blocks);
     h_lens.assign(nm, -1);
     for (int64_t m = 0; m < nm; ++m)
@@ -747,8 +752,6 @@ struct LmEngine {
         h_lens[m] = (int32_t)(ctx.h_blk0[m] + (ctx.h_cam0[m + 1] - ctx.h_cam0[m]));
     detail::h2d(lens_row, h_lens, s);
     lens_pos.alloc(detail::at_least_1(nb), s);
-    bar.alloc(nm, s);
-    bar_base.alloc(nm, s);
     if (implicit) {
       choose_point_variant();
       setup_implicit();
@@ -899,9 +902,11 @@ struct LmEngine {
     check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, implicit_kernel(), kPcgThreads, 0),
           "occupancy");
     imp_ncta = std::min(std::max(1, occ) * ctx.n_sm, kMaxGroupCtas);
+    bar.alloc(ctx.nm, s), bar_base.alloc(ctx.nm, s);
     bar.zero();
     bar_base.zero();
     pcg_part.alloc(kParts * (size_t)imp_ncta, s);
+    z.alloc(detail::at_least_1(ctx.nb) * 6, s), p.alloc(detail::at_least_1(ctx.nb) * 12, s);
     ia = ImpArgs<R>{bar, bar_base, pcg_part, imp_ncta, ctx.err, P, SV, B.Z, Zl, kept, own, camX,
                     pre, g, x, rbuf, z, p, qbuf, tbuf, h_lens[0], (int32_t)ctx.nb, pcg_iters,
                     pcg_limit, o.pcg_tol, o.wait_limit};
@@ -920,12 +925,18 @@ struct LmEngine {
     plan = detail::plan_pcg(ctx, SB.h_row_ptr, h_lens, max_ctas, rows_target, (int)smem_rows);
     detail::h2d(jobs, plan.jobs, s);
     detail::h2d(cta_job0, plan.cta_job0, s);
-    bar.zero();
-    bar_base.zero();
-    pcg_part.alloc(kParts * (size_t)plan.ncta, s);
+    // Sequence numbers start at 0 in every word; a launch's first is 1.
+    pcg_epoch.alloc(ctx.nm, s), pcg_words.alloc(3 * kPartPitch * (size_t)plan.ncta, s);
+    pcg_zx.alloc(detail::at_least_1(ctx.nb) * kZRowWords, s);
+    pcg_said.alloc(3 * kSaidPitch * (size_t)ctx.nm, s);
+    pcg_epoch.zero(), pcg_words.zero(), pcg_said.zero(), pcg_zx.zero();
+    uint32_t most = 0;
+    for (const PcgJob& j : plan.jobs)
+      most = std::max(most, pcg_blocks(SB.h_row_ptr.data(), j, h_lens[j.model]));
+    pblk.alloc(most > smem_blocks ? (size_t)SB.nz * 6 : 1, s);
     check(cudaStreamSynchronize(s), "sync");  // host plan vectors
-    pa = PcgArgs<R>{jobs, cta_job0, bar, bar_base, pcg_part, plan.ncta, SB.row_ptr, SB.col_idx,
-                    S, pre, g, x, z, p, ctx.nb, lens_row, lens_pos, SB.diag_pos, smem_rows,
+    pa = PcgArgs<R>{jobs, cta_job0, pcg_epoch, pcg_words, pcg_said, pcg_zx, plan.ncta, SB.row_ptr,
+                    SB.col_idx, S, pre, g, x, pblk, lens_row, lens_pos, SB.diag_pos, smem_rows,
                     smem_blocks, active, pcg_iters, pcg_limit, o.pcg_tol, ctx.err,
                     o.wait_limit, o.hold_cta};
     pa.cap = pcg_cap;
