@@ -12,10 +12,9 @@
 //  * points as f32, rounded to nearest.
 //
 // Observations are grouped by camera with one stable radix sort; a CTA per
-// camera walks its observations' points and counts co-observing cameras in
-// a shared-memory histogram (global scratch when the camera count does not
-// fit), then picks the top entries by CTA-wide argmax. Depths are sorted
-// within each camera by two stable radix sorts (depth bits, then camera).
+// camera walks its observations' points, counts co-observing cameras in a
+// shared-memory histogram (global scratch when the camera count does not
+// fit), picks the top entries by CTA-wide argmax, and selects the two depths.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -23,11 +22,12 @@
 #include "ba_gb300.h"
 #include "context.cuh"
 #include "primitives.cuh"
+#include "select.cuh"
 
 namespace ba {
 namespace {
 
-constexpr int kNbThreads = 256;
+constexpr int kNbThreads = 512;
 constexpr int kMaxNeighbours = 64;
 constexpr int64_t kSmemHistCams = 24576;  // 96 KB of u32 counts
 
@@ -45,59 +45,6 @@ __global__ void cam_keys_kernel(int64_t no, const uint32_t* obs_cam, uint64_t* k
   if (i >= no) return;
   key[i] = obs_cam[i];
   idx[i] = (uint32_t)i;
-}
-
-// f64 bits -> u64 whose unsigned order is f64::total_cmp's order.
-__device__ __forceinline__ uint64_t total_order_key(double z) {
-  const uint64_t b = (uint64_t)__double_as_longlong(z);
-  return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double from_total_order_key(uint64_t k) {
-  const uint64_t b = (k >> 63) ? (k & 0x7fffffffffffffffull) : ~k;
-  return __longlong_as_double((long long)b);
-}
-
-// Camera-frame depth of every observation, (R (X - C)).z with the products
-// summed left to right and no fused multiply-add (Pose::to_cam,
-// geometry.rs:57-59, as sparse.rs:476 uses it).
-__global__ void depth_keys_kernel(int64_t no, const uint32_t* obs_cam, const uint32_t* obs_pt,
-                                  const double* rot, const double* center, const double* points,
-                                  uint64_t* dkey, uint32_t* dcam) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= no) return;
-  const uint32_t c = obs_cam[i], p = obs_pt[i];
-  const double* R = rot + 9 * (size_t)c + 6;
-  const double* C = center + 3 * (size_t)c;
-  const double* X = points + 3 * (size_t)p;
-  const double d0 = __dsub_rn(X[0], C[0]), d1 = __dsub_rn(X[1], C[1]),
-               d2 = __dsub_rn(X[2], C[2]);
-  const double z = __dadd_rn(__dadd_rn(__dmul_rn(R[0], d0), __dmul_rn(R[1], d1)),
-                             __dmul_rn(R[2], d2));
-  dkey[i] = total_order_key(z);
-  dcam[i] = c;
-}
-
-// (depth key, camera) -> (camera, depth key) for the second, stable sort.
-__global__ void swap_keys_kernel(int64_t n, const uint64_t* dkey, const uint32_t* dcam,
-                                 uint64_t* ckey, uint64_t* cval) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  ckey[i] = dcam[i];
-  cval[i] = dkey[i];
-}
-
-__global__ void depth_range_kernel(int64_t nc, const uint32_t* cam_ptr, const uint64_t* sorted,
-                                   double agl, double* range) {
-  const int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= nc) return;
-  const uint32_t b = cam_ptr[a], n = cam_ptr[a + 1] - b;
-  if (n >= 10) {
-    range[2 * a] = from_total_order_key(sorted[b + n / 20]) * 0.8;
-    range[2 * a + 1] = from_total_order_key(sorted[b + (uint64_t)n * 19 / 20]) * 1.25;
-  } else {
-    range[2 * a] = agl * 0.3;
-    range[2 * a + 1] = agl * 3.0;
-  }
 }
 
 __device__ __forceinline__ uint64_t block_max_u64(uint64_t v, uint64_t* red) {
@@ -118,40 +65,86 @@ __device__ __forceinline__ uint64_t block_max_u64(uint64_t v, uint64_t* red) {
   return r;
 }
 
-struct NbArgs {
+struct CamArgs {
   int64_t nc;
   const uint32_t* cam_ptr;  // [nc + 1] into cam_obs
   const uint32_t* cam_obs;  // observation indices grouped by camera
   const uint32_t* pt_ptr;   // [np + 1] into the (point-sorted) observations
   const uint32_t* obs_cam;
   const uint32_t* obs_pt;
+  const double* rot;
+  const double* center;
+  const double* points;
+  double agl;
   int max_nb;
   uint32_t* hist_global;  // gridDim.x * nc counts when not in shared memory
+  uint64_t* key_global;   // [n_obs] depth keys of cameras beyond kDepthKeys
   uint32_t* nb;           // [nc * max_nb], UINT32_MAX padded
   uint32_t* shared;       // [nc * max_nb], 0 padded
   int32_t* n_nb;          // [nc]
+  double* range;          // [nc * 2]
 };
 
-// Persistent CTAs, one camera at a time: count the cameras that observe the
-// points this camera observes (sparse.rs:477-481: every ordered pair of
-// distinct cameras of a point), then take the largest counts.
+constexpr uint32_t kDepthKeys = 8192;  // depth keys of a camera in shared memory
+
+// Camera-frame depth of a point, (R (X - C)).z with the products summed left
+// to right and no fused multiply-add (Pose::to_cam, geometry.rs:57-59, as
+// sparse.rs:476 uses it).  R: the third row.
+__device__ __forceinline__ double depth_of(const double* R, const double* C, const double* X) {
+  const double d0 = __dsub_rn(X[0], C[0]), d1 = __dsub_rn(X[1], C[1]),
+               d2 = __dsub_rn(X[2], C[2]);
+  return __dadd_rn(__dadd_rn(__dmul_rn(R[0], d0), __dmul_rn(R[1], d1)), __dmul_rn(R[2], d2));
+}
+
+// Persistent CTAs, one camera at a time, a thread per observation of the
+// camera: the point's depth, and a count for every other camera of the point
+// (sparse.rs:477-481: every ordered pair of distinct cameras of a point);
+// then the largest counts by CTA-wide argmax, and the two depths of the range
+// by selection (sparse.rs:519-525).
+//
+// Bound by the latency of the gathers (observation, point, track).  A warp
+// per observation, its lanes over the six or seven cameras of the point, left
+// 25 of 32 lanes idle (1.34 ms for 3.0 million observations of 500 cameras);
+// the depths were sorted over all cameras, by value and then by camera, in
+// nine passes (0.75 ms).
 template <bool kSmem>
-__global__ void __launch_bounds__(kNbThreads) neighbours_kernel(NbArgs A) {
-  extern __shared__ uint32_t smem_hist[];
+__global__ void __launch_bounds__(kNbThreads) camera_summary_kernel(CamArgs A) {
+  extern __shared__ __align__(8) unsigned char smem_raw[];
   __shared__ uint64_t red[kNbThreads / 32 + 1];
-  uint32_t* hist = kSmem ? smem_hist : A.hist_global + (size_t)blockIdx.x * A.nc;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ uint32_t bytes[256], found[3];
+  uint64_t* skey = reinterpret_cast<uint64_t*>(smem_raw);
+  uint32_t* hist = kSmem ? reinterpret_cast<uint32_t*>(skey + kDepthKeys)
+                         : A.hist_global + (size_t)blockIdx.x * A.nc;
   for (int64_t c = threadIdx.x; c < A.nc; c += kNbThreads) hist[c] = 0;
   __syncthreads();
   for (int64_t a = blockIdx.x; a < A.nc; a += gridDim.x) {
-    for (uint32_t k = A.cam_ptr[a] + warp; k < A.cam_ptr[a + 1]; k += kNbThreads / 32) {
-      const uint32_t p = A.obs_pt[A.cam_obs[k]];
-      for (uint32_t j = A.pt_ptr[p] + lane; j < A.pt_ptr[p + 1]; j += 32) {
-        const uint32_t b = A.obs_cam[j];
-        if (b != (uint32_t)a) atomicAdd(&hist[b], 1u);
+    const uint32_t b = A.cam_ptr[a], n = A.cam_ptr[a + 1] - b;
+    uint64_t* key = n <= kDepthKeys ? skey : A.key_global + b;
+    const double R[3] = {A.rot[9 * a + 6], A.rot[9 * a + 7], A.rot[9 * a + 8]};
+    const double C[3] = {A.center[3 * a], A.center[3 * a + 1], A.center[3 * a + 2]};
+    for (uint32_t i = threadIdx.x; i < n; i += kNbThreads) {
+      const uint32_t p = A.obs_pt[A.cam_obs[b + i]];
+      key[i] = total_order_key(depth_of(R, C, A.points + 3 * (size_t)p));
+      const uint32_t e = A.pt_ptr[p + 1];
+#pragma unroll 4
+      for (uint32_t j = A.pt_ptr[p]; j < e; ++j) {
+        const uint32_t o = A.obs_cam[j];
+        if (o != (uint32_t)a) atomicAdd(&hist[o], 1u);
       }
     }
     __syncthreads();
+    if (n >= 10) {
+      const uint64_t lo = select_key<kNbThreads>(key, n, n / 20, bytes, found);
+      const uint64_t hi =
+          select_key<kNbThreads>(key, n, (uint32_t)((uint64_t)n * 19 / 20), bytes, found);
+      if (threadIdx.x == 0) {
+        A.range[2 * a] = from_total_order_key(lo) * 0.8;
+        A.range[2 * a + 1] = from_total_order_key(hi) * 1.25;
+      }
+    } else if (threadIdx.x == 0) {
+      A.range[2 * a] = A.agl * 0.3;
+      A.range[2 * a + 1] = A.agl * 3.0;
+    }
     int r = 0;
     for (; r < A.max_nb; ++r) {
       uint64_t best = 0;
@@ -161,11 +154,11 @@ __global__ void __launch_bounds__(kNbThreads) neighbours_kernel(NbArgs A) {
       }
       best = block_max_u64(best, red);
       if (best == 0) break;
-      const uint32_t b = 0xffffffffu - (uint32_t)best;
+      const uint32_t o = 0xffffffffu - (uint32_t)best;
       if (threadIdx.x == 0) {
-        A.nb[a * A.max_nb + r] = b;
+        A.nb[a * A.max_nb + r] = o;
         A.shared[a * A.max_nb + r] = (uint32_t)(best >> 32);
-        hist[b] = 0;
+        hist[o] = 0;
       }
       __syncthreads();
     }
@@ -227,34 +220,21 @@ struct SummaryRun {
       if (nc > 0) lower_bounds_u64(key, no, cam_ptr, nc, 1, s);
     }
     if (nc > 0) {
-      // Depths sorted within each camera: by total order, then (stably) by camera.
-      DevBuf<uint64_t> dkey(std::max<int64_t>(no, 1), s), dtmp(std::max<int64_t>(no, 1), s);
-      DevBuf<uint32_t> dcam(std::max<int64_t>(no, 1), s), ctmp(std::max<int64_t>(no, 1), s);
-      if (no > 0) {
-        BA_LAUNCH(depth_keys_kernel<<<grid_for(no, 256), 256, 0, s>>>(no, obs_cam, obs_pt, rot, center,
-                                                                     points, dkey, dcam));
-        radix_sort_u64_u32(dkey, dcam, dtmp, ctmp, no, 64, s);
-      }
-      DevBuf<uint64_t> ckey(std::max<int64_t>(no, 1), s), cval(std::max<int64_t>(no, 1), s);
-      if (no > 0) {
-        BA_LAUNCH(swap_keys_kernel<<<grid_for(no, 256), 256, 0, s>>>(no, dkey, dcam, ckey, cval));
-        // The sort scratch of the first sort is reused for the second.
-        radix_sort_u64_u64(ckey, cval, dtmp, dkey, no, bit_width(nc), s);
-      }
-      BA_LAUNCH(depth_range_kernel<<<grid_for(nc, 128), 128, 0, s>>>(nc, cam_ptr, cval, agl, range));
       const bool in_smem = nc <= kSmemHistCams;
-      const unsigned grid = (unsigned)std::min<int64_t>(nc, 2 * (int64_t)std::max(n_sm, 1));
+      const size_t smem = kDepthKeys * 8 + (in_smem ? (size_t)nc * 4 : 0);
+      auto kernel = in_smem ? camera_summary_kernel<true> : camera_summary_kernel<false>;
+      check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+            "summary smem");
+      int occ = 0;
+      check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kNbThreads, smem),
+            "occupancy");
+      const unsigned grid =
+          (unsigned)std::min<int64_t>(nc, (int64_t)std::max(occ, 1) * std::max(n_sm, 1));
       if (!in_smem) A(hist, (int64_t)grid * nc);
-      NbArgs na{nc, cam_ptr, cam_obs, pt_ptr, obs_cam, obs_pt, max_nb, hist, nb, shared, n_nb};
-      if (in_smem) {
-        const size_t smem = (size_t)nc * 4;
-        check(cudaFuncSetAttribute(neighbours_kernel<true>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-              "neighbours smem");
-        BA_LAUNCH(neighbours_kernel<true><<<grid, kNbThreads, smem, s>>>(na));
-      } else {
-        BA_LAUNCH(neighbours_kernel<false><<<grid, kNbThreads, 0, s>>>(na));
-      }
+      DevBuf<uint64_t> key(no > (int64_t)kDepthKeys ? no : 1, s);
+      CamArgs ca{nc,     cam_ptr, cam_obs, pt_ptr, obs_cam, obs_pt, rot,  center, points,
+                 agl,    max_nb,  hist,    key,    nb,      shared, n_nb, range};
+      BA_LAUNCH(kernel<<<grid, kNbThreads, smem, s>>>(ca));
     }
     if (np > 0) BA_LAUNCH(points_f32_kernel<<<grid_for(3 * np, 256), 256, 0, s>>>(3 * np, points, pts32));
   }
