@@ -1,0 +1,47 @@
+// Intrinsics::undistort (geometry.rs:35-44) for the device passes: pixel to
+// normalised coordinates by eight fixed-point steps x <- q / d(x).
+//
+// The steps are FP64 operations one after the other, ~64 cycles of the SM
+// sub-partition each, and a division is nine of them; the two of a step share
+// their divisor.  So a step takes one reciprocal (five) and two residual
+// corrections (three each): 16 operations instead of 23 with the polynomial.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace ba {
+
+static __device__ __noinline__ double quotient_slow(double x, double d) { return x / d; }
+
+// x / d with r = 1 / d rounded to nearest: q = x r and one residual
+// correction, which rounds x / d + (x / d - q)(1 - d r), i.e. the quotient but
+// for 2^-52 of a last place (Markstein, IBM J. Res. Dev. 34, 1990).  The
+// residual is exact where neither it nor q leaves the normal range; outside
+// of 2^-900 .. 2^900 (and for zero, infinite or NaN values) the division.
+__device__ __forceinline__ double quotient_by(double x, double d, double r) {
+  const double q = x * r;
+  const uint32_t eq = ((uint32_t)__double2hiint(q) >> 20) & 0x7ffu;
+  const uint32_t er = ((uint32_t)__double2hiint(r) >> 20) & 0x7ffu;
+  if (eq - 123u > 1800u || er - 123u > 1800u) return quotient_slow(x, d);
+  return fma(fma(-q, d, x), r, q);
+}
+
+// K = {f, cx, cy, k1, k2}; rf = 1 / f rounded to nearest.
+__device__ __forceinline__ void undistort(const double* K, double rf, double u, double v,
+                                          double* p) {
+  const double f = K[0], k1 = K[3], k2 = K[4];
+  const double qx = quotient_by(u - K[1], f, rf), qy = quotient_by(v - K[2], f, rf);
+  double px = qx, py = qy;
+#pragma unroll 1
+  for (int i = 0; i < 8; ++i) {
+    const double r2 = px * px + py * py;
+    const double d = 1.0 + k1 * r2 + k2 * r2 * r2;
+    const double r = __drcp_rn(d);
+    px = quotient_by(qx, d, r);
+    py = quotient_by(qy, d, r);
+  }
+  p[0] = px, p[1] = py;
+}
+
+}  // namespace ba

@@ -1,14 +1,16 @@
-"""GPU: order statistics selected inside a CTA (depth ranges of the summary)
-at the sizes where they can go wrong: the ranks' edges, keys
+"""GPU: order statistics selected inside a CTA (depth ranges of the summary,
+pair medians) at the sizes where they can go wrong: the ranks' edges, keys
 that fill shared memory or exceed it by one, equal values, one value.
 
-The summary's depths are bit-exact (no fused operation on either side)."""
+The summary's depths are bit-exact (no fused operation on either side); the
+medians keep the bound of the other pair check tests (1e-9 of the largest:
+the oracle's Sampson error differs by fused operations)."""
 import numpy as np
 import pytest
 
 import ba_oracle as O
 import stitch_ba
-from stitch_ba import Problem
+from stitch_ba import PairMatches, Problem, survey
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +37,23 @@ def test_depth_ranges_match_oracle(sizes, levels):
     nb, _, _, depth_range, _ = O.sparse_summary(oc, op, R, C, X, agl=80.0)
     assert np.array_equal(out.depth_range, depth_range)
     assert np.array_equal(out.neighbours, nb)
+
+
+@pytest.mark.parametrize("sizes", [(1, 2, 3, 0, 255, 256, 257), (3071, 3072, 3073, 9000),
+                                   (700_000, 5, 400_000)])
+def test_pair_medians_match_oracle(sizes):
+    """Up to the pairs that go through global memory, and a call large enough
+    to be copied in two pieces (1.1 million matches)."""
+    rng = np.random.default_rng(len(sizes))
+    p, _ = survey.generate("lawnmower77", seed=3, n_cams=8, n_points=400)
+    n = sum(sizes)
+    uv = rng.uniform([0, 0, 0, 0], [5472, 3648, 5472, 3648], (n, 4))
+    uv[::5] = uv[0]                        # equal errors
+    uv[1::7, :2] = p.intr[0, 1:3]          # the principal point: a zero quotient
+    pairs = np.array([(i, i + 1) for i in range(len(sizes))], np.uint32)
+    ptr = np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint32)
+    med = stitch_ba.pair_fits(PairMatches(pairs, ptr, uv), p.rot, p.center, p.intr, p.cam_group)
+    ref = O.pair_fits(pairs, ptr, uv, p.rot, p.center, p.intr, p.cam_group)
+    some = np.array(sizes) > 0
+    assert np.abs(med - ref)[some].max() <= 1e-9 * np.abs(ref[some]).max()
+    assert np.array_equal(med[~some], ref[~some])
