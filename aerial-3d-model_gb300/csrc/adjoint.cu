@@ -22,20 +22,66 @@ namespace {
 
 constexpr unsigned T = 256;
 
-// Per observation: pred Jacobians in FP64 (rows u, v): jc 2x6, jp 2x3,
-// ji 2x5 (f, cx, cy, k1, k2), residual e, weight w; false if behind.
-__device__ bool full_jacobian(const Prob& P, const StateView& st, int64_t k, double sigma,
-                              double* jc, double* jp, double* ji, double* e, double* w) {
-  double o[kLinW];
-  if (!linearise<double>(P, st, k, sigma, true, o)) return false;
-  for (int i = 0; i < 12; ++i) jc[i] = o[i];
-  for (int i = 0; i < 6; ++i) jp[i] = o[12 + i];
-  // intrinsics: (f, cx, cy, k1, k2); linearise gives d/d(f, k1, k2)
-  ji[0] = o[18], ji[1] = 1.0, ji[2] = 0.0, ji[3] = o[19], ji[4] = o[20];
-  ji[5] = o[21], ji[6] = 0.0, ji[7] = 1.0, ji[8] = o[22], ji[9] = o[23];
-  e[0] = o[24], e[1] = o[25];
-  *w = o[26];
-  return true;
+// One observation's share of the VJP, in reverse mode: the cotangent goes
+// back through the projection once instead of through Jacobian rows (63 FP64
+// operations, 15 more where the cotangent is the cost's; the rows took 171).
+struct ObsVjp {
+  double rot[3];  // left perturbation of the rotation
+  double pt[3];   // point; the centre's share is its negative
+  double in[5];   // f, cx, cy, k1, k2
+};
+
+// cot: the caller's residual cotangents [2n], or null: those of the robust
+// cost.  kGeo: rotation and point too.  Zero for an observation that is not
+// in front of its camera.
+template <bool kGeo>
+__device__ __forceinline__ void obs_vjp(const Prob& P, const StateView& st, int64_t k, double sigma,
+                                        const double* cot, ObsVjp& o) {
+  const uint32_t cam = P.obs_cam[k];
+  const double* R = st.rot + 9 * (size_t)cam;
+  const double* K = st.intr + 5 * (size_t)P.cam_group[cam];
+  double xc[3];
+  bacam::to_cam(R, st.center + 3 * (size_t)cam, st.points + 3 * (size_t)P.obs_pt[k], xc);
+  if (xc[2] <= 1e-6) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) o.rot[i] = o.pt[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) o.in[i] = 0.0;
+    return;
+  }
+  const double f = K[0], k1 = K[3], k2 = K[4];
+  const double iz = __drcp_rn(xc[2]);
+  const double px = xc[0] * iz, py = xc[1] * iz;
+  const double r2 = px * px + py * py;
+  const double d = 1.0 + k1 * r2 + k2 * r2 * r2;
+  const double qx = px * d, qy = py * d;
+  // e = u - pred: the prediction's cotangent is the residual's negative
+  double l0, l1;
+  if (cot) {
+    l0 = -cot[2 * k], l1 = -cot[2 * k + 1];
+  } else {  // d rho / d e = rho'(|e|^2) * 2 e, rho' = the IRLS weight
+    const double ex = P.obs_uv[2 * k] - (f * qx + K[1]);
+    const double ey = P.obs_uv[2 * k + 1] - (f * qy + K[2]);
+    const double w = -2.0 * robust_weight(ex * ex + ey * ey, sigma, P.loss);
+    l0 = w * ex, l1 = w * ey;
+  }
+  const double s = l0 * px + l1 * py;
+  o.in[0] = l0 * qx + l1 * qy;
+  o.in[1] = l0;
+  o.in[2] = l1;
+  o.in[3] = f * r2 * s;
+  o.in[4] = o.in[3] * r2;
+  if constexpr (kGeo) {
+    const double cs = 2.0 * (k1 + 2.0 * k2 * r2) * s;
+    const double fz = f * iz;
+    const double g0 = (d * l0 + cs * px) * fz, g1 = (d * l1 + cs * py) * fz;
+    const double g2 = -(g0 * px + g1 * py);
+    o.rot[0] = xc[1] * g2 - xc[2] * g1;
+    o.rot[1] = xc[2] * g0 - xc[0] * g2;
+    o.rot[2] = xc[0] * g1 - xc[1] * g0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) o.pt[j] = R[j] * g0 + R[3 + j] * g1 + R[6 + j] * g2;
+  }
 }
 
 __global__ void linearise_all_kernel(Prob P, StateView st, double sigma, double* out,
@@ -48,33 +94,6 @@ __global__ void linearise_all_kernel(Prob P, StateView st, double sigma, double*
     for (int i = 0; i < kLinW; ++i) o[i] = 0.0;
 }
 
-// Per observation VJP contributions: camera (6), point (3), intrinsics (5).
-// cot: caller's residual cotangents [2n], or null for the cost gradient.
-__global__ void vjp_obs_kernel(Prob P, StateView st, double sigma, const double* cot,
-                               double* gcam, double* gpt, double* gint) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= P.no) return;
-  double jc[12], jp[6], ji[10], e[2], w;
-  double* c6 = gcam + 6 * (size_t)k;
-  double* p3 = gpt + 3 * (size_t)k;
-  double* i5 = gint + 5 * (size_t)k;
-  if (!full_jacobian(P, st, k, sigma, jc, jp, ji, e, &w)) {
-    for (int i = 0; i < 6; ++i) c6[i] = 0.0;
-    for (int i = 0; i < 3; ++i) p3[i] = 0.0;
-    for (int i = 0; i < 5; ++i) i5[i] = 0.0;
-    return;
-  }
-  double l0, l1;
-  if (cot) {
-    l0 = cot[2 * k], l1 = cot[2 * k + 1];
-  } else {  // d rho / d e = rho'(|e|^2) * 2 e, rho' = the IRLS weight
-    l0 = 2.0 * w * e[0], l1 = 2.0 * w * e[1];
-  }
-  for (int i = 0; i < 6; ++i) c6[i] = -(jc[i] * l0 + jc[6 + i] * l1);
-  for (int i = 0; i < 3; ++i) p3[i] = -(jp[i] * l0 + jp[3 + i] * l1);
-  for (int i = 0; i < 5; ++i) i5[i] = -(ji[i] * l0 + ji[5 + i] * l1);
-}
-
 // Thread per point: its observations' contributions in order.
 __global__ void vjp_point_kernel(Prob P, const uint32_t* pt_ptr, const double* gpt, double* out) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -85,33 +104,100 @@ __global__ void vjp_point_kernel(Prob P, const uint32_t* pt_ptr, const double* g
   for (int i = 0; i < 3; ++i) out[3 * p + i] = a[i];
 }
 
-// CTA per camera: observations in camera order, plus the prior term.
-__global__ void __launch_bounds__(128)
+// A quarter of a camera's observations per CTA, in camera order: their shares
+// of the camera and its intrinsics summed, the points' stored (24 bytes an
+// observation; with a pass of its own per observation, 112 and read again).
+// Bound by the FP64 operations; quarters, because 500 cameras on 152 SMs would
+// leave the last wave a third full.
+constexpr int kVjpThreads = 128;
+constexpr int kVjpParts = 4;
+constexpr int kVjpN = 11;  // rotation 3, centre 3, intrinsics 5
+
+__global__ void __launch_bounds__(kVjpThreads)
     vjp_camera_kernel(Prob P, StateView st, const uint32_t* cam_ptr, const uint32_t* cam_obs,
-                      const double* gcam, const double* gint, const double* cot_prior,
-                      double* out_cam, double* out_cam_int) {
-  __shared__ double scratch[11 * 32];
-  const int64_t c = blockIdx.x;
-  double a[11];
-  for (int i = 0; i < 11; ++i) a[i] = 0.0;
-  for (uint32_t i = cam_ptr[c] + threadIdx.x; i < cam_ptr[c + 1]; i += blockDim.x) {
+                      double sigma, const double* cot, double* gpt, double* part) {
+  __shared__ double scratch[kVjpN * 32];
+  const int64_t c = blockIdx.x / kVjpParts, q = blockIdx.x % kVjpParts;
+  const uint32_t c0 = cam_ptr[c], n = cam_ptr[c + 1] - c0;
+  const uint32_t b = c0 + (uint32_t)((uint64_t)n * q / kVjpParts);
+  const uint32_t e = c0 + (uint32_t)((uint64_t)n * (q + 1) / kVjpParts);
+  double a[kVjpN];
+#pragma unroll
+  for (int i = 0; i < kVjpN; ++i) a[i] = 0.0;
+  for (uint32_t i = b + threadIdx.x; i < e; i += kVjpThreads) {
     const uint32_t k = cam_obs[i];
-    for (int t = 0; t < 6; ++t) a[t] += gcam[6 * (size_t)k + t];
-    for (int t = 0; t < 5; ++t) a[6 + t] += gint[5 * (size_t)k + t];
+    ObsVjp o;
+    obs_vjp<true>(P, st, k, sigma, cot, o);
+    if (gpt)
+#pragma unroll
+      for (int t = 0; t < 3; ++t) gpt[3 * (size_t)k + t] = o.pt[t];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) a[t] += o.rot[t], a[3 + t] -= o.pt[t];
+#pragma unroll
+    for (int t = 0; t < 5; ++t) a[6 + t] += o.in[t];
   }
-  block_sum<11>(a, scratch);
-  if (threadIdx.x == 0) {
-    if (P.prior_mask && P.prior_mask[c]) {
-      const double* q = P.prior + 6 * (size_t)c;
-      for (int t = 0; t < 3; ++t) {
-        const double r = (st.center[3 * c + t] - q[t]) / q[3 + t];
-        const double mu = cot_prior ? cot_prior[3 * c + t] : 2.0 * r;
-        a[3 + t] += mu / q[3 + t];
-      }
+  block_sum<kVjpN>(a, scratch);
+  if (threadIdx.x == 0)
+    for (int t = 0; t < kVjpN; ++t) part[(size_t)blockIdx.x * kVjpN + t] = a[t];
+}
+
+// Thread per camera: its quarters in order, plus the prior term.
+__global__ void vjp_camera_sum_kernel(Prob P, StateView st, const double* part,
+                                      const double* cot_prior, double* out_cam,
+                                      double* out_cam_int) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= P.nc) return;
+  double a[kVjpN];
+#pragma unroll
+  for (int t = 0; t < kVjpN; ++t) {
+    a[t] = 0.0;
+    for (int q = 0; q < kVjpParts; ++q) a[t] += part[(size_t)(kVjpParts * c + q) * kVjpN + t];
+  }
+  if (P.prior_mask && P.prior_mask[c]) {
+    const double* q = P.prior + 6 * (size_t)c;
+    for (int t = 0; t < 3; ++t) {
+      const double r = (st.center[3 * c + t] - q[t]) / q[3 + t];
+      const double mu = cot_prior ? cot_prior[3 * c + t] : 2.0 * r;
+      a[3 + t] += mu / q[3 + t];
     }
-    for (int t = 0; t < 6; ++t) out_cam[6 * c + t] = a[t];
-    for (int t = 0; t < 5; ++t) out_cam_int[5 * c + t] = a[6 + t];
   }
+#pragma unroll
+  for (int t = 0; t < 6; ++t) out_cam[6 * c + t] = a[t];
+#pragma unroll
+  for (int t = 0; t < 5; ++t) out_cam_int[5 * c + t] = a[6 + t];
+}
+
+// Intrinsics alone, models of one lens group each: a chunk of a model's
+// observations per CTA, in observation order (no index by camera is built),
+// then a model's chunks by a CTA.
+__global__ void __launch_bounds__(kCostThreads)
+    vjp_chunk_kernel(Prob P, StateView st, StructView S, double sigma, const double* cot,
+                     double* part) {
+  __shared__ double scratch[5 * 32];
+  double a[5] = {0, 0, 0, 0, 0};
+  for (uint32_t k = S.cost_chunk_begin[blockIdx.x] + threadIdx.x;
+       k < S.cost_chunk_end[blockIdx.x]; k += kCostThreads) {
+    ObsVjp o;
+    obs_vjp<false>(P, st, k, sigma, cot, o);
+#pragma unroll
+    for (int t = 0; t < 5; ++t) a[t] += o.in[t];
+  }
+  block_sum<5>(a, scratch);
+  if (threadIdx.x == 0)
+    for (int t = 0; t < 5; ++t) part[5 * (size_t)blockIdx.x + t] = a[t];
+}
+
+__global__ void __launch_bounds__(kCostFinalThreads)
+    vjp_chunk_sum_kernel(StructView S, const double* part, const uint32_t* group, double* out) {
+  __shared__ double scratch[5 * 32];
+  const int64_t m = blockIdx.x;
+  double a[5] = {0, 0, 0, 0, 0};
+  for (uint32_t c = S.model_chunk0[m] + threadIdx.x; c < S.model_chunk0[m + 1];
+       c += kCostFinalThreads)
+    for (int t = 0; t < 5; ++t) a[t] += part[5 * (size_t)c + t];
+  block_sum<5>(a, scratch);
+  if (threadIdx.x == 0 && group[m + 1] > group[m])
+    for (int t = 0; t < 5; ++t) out[5 * (size_t)group[m] + t] = a[t];
 }
 
 __global__ void vjp_group_kernel(Prob P, const uint32_t* grp_ptr, const uint32_t* grp_cams,
@@ -230,26 +316,45 @@ void context_vjp(Context& c, const ba_options* opt, const double* cot_obs,
   cudaStream_t s = c.stream;
   const Prob P = c.prob(o.loss);
   const int64_t no = c.no, nc = c.nc, np = c.np, ng = c.ng;
-  StructBufs SB;
-  SB.pt_ptr.alloc(np + 1, s);
-  lower_bounds_u32(P.obs_pt, no, SB.pt_ptr, np, s);
-  build_cam_index(P, SB, s);
   DevBuf<double> d_cot(cot_obs ? 2 * no : 0, s), d_cotp(cot_prior ? 3 * nc : 0, s);
   if (cot_obs && no)
     check(cudaMemcpyAsync(d_cot.p, cot_obs, 16 * no, cudaMemcpyHostToDevice, s), "h2d");
   if (cot_prior && nc)
     check(cudaMemcpyAsync(d_cotp.p, cot_prior, 24 * nc, cudaMemcpyHostToDevice, s), "h2d");
-  DevBuf<double> gc(std::max<int64_t>(no, 1) * 6, s), gp(std::max<int64_t>(no, 1) * 3, s),
-      gi(std::max<int64_t>(no, 1) * 5, s);
+  const double* cot = cot_obs ? d_cot.p : nullptr;
+  DevBuf<double> og(std::max<int64_t>(ng, 1) * 5, s);
+  bool one_group = true;
+  for (int64_t m = 0; m < c.nm; ++m) one_group = one_group && c.h_grp0[m + 1] - c.h_grp0[m] <= 1;
+  if (!g_cam && !g_pt && one_group) {
+    CostPlan pl;
+    make_cost_plan(c, pl);
+    DevBuf<double> part(5 * (size_t)pl.n, s);
+    DevBuf<uint32_t> grp0(c.nm + 1, s);
+    check(cudaMemcpyAsync(grp0.p, c.h_grp0.data(), 4 * (c.nm + 1), cudaMemcpyHostToDevice, s), "h2d");
+    BA_LAUNCH(vjp_chunk_kernel<<<(unsigned)pl.n, kCostThreads, 0, s>>>(P, c.cur(), pl.view(),
+                                                                      o.sigma, cot, part));
+    BA_LAUNCH(vjp_chunk_sum_kernel<<<(unsigned)c.nm, kCostFinalThreads, 0, s>>>(pl.view(), part,
+                                                                               grp0, og));
+    if (g_intr && ng) check(cudaMemcpyAsync(g_intr, og.p, 40 * ng, cudaMemcpyDeviceToHost, s), "d2h");
+    check(cudaStreamSynchronize(s), "vjp");
+    return;
+  }
+  StructBufs SB;
+  build_cam_index(P, SB, s);
+  DevBuf<double> gp(std::max<int64_t>(g_pt ? 3 * no : 1, 1), s);
   DevBuf<double> oc(std::max<int64_t>(nc, 1) * 6, s), oci(std::max<int64_t>(nc, 1) * 5, s),
-      op(std::max<int64_t>(np, 1) * 3, s), og(std::max<int64_t>(ng, 1) * 5, s);
-  if (no)
-    BA_LAUNCH(vjp_obs_kernel<<<grid_for(no, T), T, 0, s>>>(P, c.cur(), o.sigma,
-                                                          cot_obs ? d_cot.p : nullptr, gc, gp, gi));
-  if (np) BA_LAUNCH(vjp_point_kernel<<<grid_for(np, T), T, 0, s>>>(P, SB.pt_ptr, gp, op));
-  if (nc)
-    BA_LAUNCH(vjp_camera_kernel<<<(unsigned)nc, 128, 0, s>>>(
-        P, c.cur(), SB.cam_ptr, SB.cam_obs, gc, gi, cot_prior ? d_cotp.p : nullptr, oc, oci));
+      part(std::max<int64_t>(nc, 1) * kVjpParts * kVjpN, s), op(std::max<int64_t>(np, 1) * 3, s);
+  if (nc) {
+    BA_LAUNCH(vjp_camera_kernel<<<(unsigned)(nc * kVjpParts), kVjpThreads, 0, s>>>(
+        P, c.cur(), SB.cam_ptr, SB.cam_obs, o.sigma, cot, g_pt ? gp.p : nullptr, part));
+    BA_LAUNCH(vjp_camera_sum_kernel<<<grid_for(nc, 128), 128, 0, s>>>(
+        P, c.cur(), part, cot_prior ? d_cotp.p : nullptr, oc, oci));
+  }
+  if (np && g_pt) {
+    SB.pt_ptr.alloc(np + 1, s);
+    lower_bounds_u32(P.obs_pt, no, SB.pt_ptr, np, s);
+    BA_LAUNCH(vjp_point_kernel<<<grid_for(np, T), T, 0, s>>>(P, SB.pt_ptr, gp, op));
+  }
   if (ng)
     BA_LAUNCH(vjp_group_kernel<<<grid_for(ng * 32, 128), 128, 0, s>>>(P, SB.grp_ptr, SB.grp_cams,
                                                                      oci, og));
