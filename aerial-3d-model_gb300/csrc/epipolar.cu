@@ -10,8 +10,8 @@
 // on one xorshift stream per pair (each draw depends on the previous), so a
 // thread per pair writes all of its pair's samples first.  Then a thread per
 // hypothesis fits the normalised 8-point F (the null vector of its 8x9
-// system, rank 2 by removing the smallest singular value); each warp counts
-// four hypotheses' inliers over the pair's correspondences (FP32 with an
+// system, rank 2 by removing the smallest singular value); a warp counts a
+// hypothesis' inliers over the pair's correspondences (FP32 with an
 // error bound, FP64 near the threshold: the decisions are the FP64 ones); a
 // CTA per pair takes the first hypothesis with the most inliers and refits on
 // its inliers (normal matrix, smallest eigenvector).  Geometry in FP64, as
@@ -32,7 +32,6 @@ namespace {
 constexpr double kF64Max = 1.7976931348623157e308;
 constexpr int kFitThreads = 64;
 constexpr int kCountThreads = 256;
-constexpr int kHypPerCountCta = 32;  // 4 hypotheses per warp
 constexpr int kRefitThreads = 128;
 constexpr int64_t kMaxChunkHyp = int64_t(1) << 22;
 
@@ -98,6 +97,7 @@ struct RansacArgs {
   double t2;
   uint32_t* samples;  // [np * iters * 8]
   double* F;          // [np * iters * 9]
+  float4* F32;        // [np * iters * 3] the same in FP32 (9 of 12 values)
   uint8_t* valid;     // [np * iters]
   int32_t* count;     // [np * iters]
   uint32_t* scratch;  // [n_matches] inlier index lists
@@ -108,50 +108,150 @@ struct RansacArgs {
   uint32_t* err;
 };
 
-__global__ void ransac_sample_kernel(RansacArgs A) {
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= A.np) return;
-  const int64_t p = A.p0 + q;
+// A pair's draws are one sequential xorshift stream, but a step of it is a
+// linear map of 64 bits, so a lane can start anywhere: lane l begins 64 l
+// steps ahead (its five bits choose among the map's powers) and draws 64
+// residues, 2048 a warp.  Samples then take eight residues each, 32 samples
+// at a time, up to the first one with a repeated index (28 / n of them), which
+// takes the distinct ones of the next 32.  A warp per pair; a thread per pair, one draw
+// after the other, held 1603 pairs of 600 samples for 0.68 ms.
+constexpr int kLaneDraws = 64;
+constexpr int kDraws = 32 * kLaneDraws;
+
+// m[k][b]: the state 64 2^k steps after the state with bit b alone.
+struct DrawJump {
+  uint64_t m[5][64];
+};
+
+__host__ __device__ __forceinline__ uint64_t xorshift64(uint64_t s) {
+  s ^= s << 13;
+  s ^= s >> 7;
+  s ^= s << 17;
+  return s;
+}
+
+const DrawJump& draw_jump() {
+  static const DrawJump j = [] {
+    DrawJump d;
+    uint64_t t[64];
+    for (int b = 0; b < 64; ++b) t[b] = xorshift64(uint64_t(1) << b);
+    auto apply = [](const uint64_t* m, uint64_t v) {
+      uint64_t r = 0;
+      for (int b = 0; b < 64; ++b)
+        if ((v >> b) & 1) r ^= m[b];
+      return r;
+    };
+    for (int e = 0; e < 11; ++e) {  // t: 2^e steps
+      if (e >= 6) std::copy(t, t + 64, d.m[e - 6]);
+      uint64_t u[64];
+      for (int b = 0; b < 64; ++b) u[b] = apply(t, t[b]);
+      std::copy(u, u + 64, t);
+    }
+    return d;
+  }();
+  return j;
+}
+
+__global__ void __launch_bounds__(32) ransac_sample_kernel(RansacArgs A,
+                                                           const __grid_constant__ DrawJump J) {
+  __shared__ uint32_t buf[2 * kDraws];  // residues not used yet
+  const int lane = threadIdx.x;
+  const int64_t q = blockIdx.x, p = A.p0 + q;
   const uint32_t n = A.match_ptr[p + 1] - A.match_ptr[p];
   if (n < 12) return;
-  uint64_t s = A.seed[p] | 1;
-  uint32_t* out = A.samples + (size_t)q * A.iters * 8;
+  uint64_t s = A.seed[p] | 1;  // state after the residues drawn so far
+  uint4* out = reinterpret_cast<uint4*>(A.samples + (size_t)q * A.iters * 8);
   // s % n without a 64-bit division: with M = floor((2^64 - 1) / n),
   // umulhi(s, M) is floor(s / n) or one less, so one correction is exact.
   const uint64_t M = ~0ull / n;
-  for (int it = 0; it < A.iters; ++it) {
-    // The eight indices stay in registers: every access below has a
-    // compile-time index (fills and duplicate checks are predicated).
-    uint32_t idx[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int k = 0;
-    // Bounded: with n >= 12 the xorshift stream yields eight distinct
-    // residues within a few dozen draws; the cap only guards the loop.
-    for (int draws = 0; k < 8; ++draws) {
-      if (draws == (1 << 20)) {
-        atomicOr(A.err, ERR_STRUCTURE);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) idx[j] = j;
-        break;
+  int have = 0, pos = 0;
+  bool more = true;
+  for (int it = 0; it < A.iters;) {
+    if (more || have - pos < 8) {
+      const int left = have - pos;
+      if (left > kDraws) {  // a sample that 2048 draws do not fill: not with n >= 12
+        if (lane == 0) atomicOr(A.err, ERR_STRUCTURE);
+        return;
       }
-      s ^= s << 13;
-      s ^= s >> 7;
-      s ^= s << 17;
-      uint64_t r = s - __umul64hi(s, M) * n;
-      if (r >= n) r -= n;
-      const uint32_t c = (uint32_t)r;
-      bool dup = false;
+      for (int i0 = 0; i0 < left; i0 += 32) {  // to the front (pos >= 32, or the buffer is empty)
+        const uint32_t v = i0 + lane < left ? buf[pos + i0 + lane] : 0u;
+        __syncwarp();
+        if (i0 + lane < left) buf[i0 + lane] = v;
+        __syncwarp();
+      }
+      uint64_t t = s;
+#pragma unroll 1
+      for (int k = 0; k < 5; ++k) {
+        uint64_t r = 0;
+#pragma unroll 8
+        for (int b = 0; b < 64; ++b) r ^= J.m[k][b] & (0ull - ((t >> b) & 1));
+        if ((lane >> k) & 1) t = r;
+      }
+#pragma unroll 4
+      for (int i = 0; i < kLaneDraws; ++i) {
+        t = xorshift64(t);
+        uint64_t r = t - __umul64hi(t, M) * n;
+        if (r >= n) r -= n;
+        buf[left + kLaneDraws * lane + i] = (uint32_t)r;
+      }
+      s = __shfl_sync(kFull, t, 31);
+      have = left + kDraws, pos = 0, more = false;
+      __syncwarp();
+    }
+    const int w = min(min(32, (have - pos) / 8), A.iters - it);
+    uint32_t idx[8];
+    bool dup = false;
+    if (lane < w) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) dup |= (j < k) & (idx[j] == c);
-      if (!dup) {
+      for (int j = 0; j < 8; ++j) idx[j] = buf[pos + 8 * lane + j];
+#pragma unroll
+      for (int j = 1; j < 8; ++j)
+#pragma unroll
+        for (int i = 0; i < j; ++i) dup |= idx[i] == idx[j];
+    }
+    const unsigned bad = __ballot_sync(kFull, dup);
+    const int first = bad ? __ffs(bad) - 1 : w;
+    if (lane < first) {
+      out[2 * (it + lane)] = make_uint4(idx[0], idx[1], idx[2], idx[3]);
+      out[2 * (it + lane) + 1] = make_uint4(idx[4], idx[5], idx[6], idx[7]);
+    }
+    it += first, pos += 8 * first;
+    if (!bad) continue;
+    // The sample with a repeated index: a lane per residue, of which it takes
+    // the first eight that no earlier lane has.
+    const uint32_t c = pos + lane < have ? buf[pos + lane] : 0xffffffffu;
+    const unsigned same = __match_any_sync(kFull, c);
+    unsigned fresh = __ballot_sync(kFull, pos + lane < have && lane == __ffs(same) - 1);
+    if (__popc(fresh) >= 8) {
+      const int rank = __popc(fresh & ((1u << lane) - 1u));
+      if (((fresh >> lane) & 1u) && rank < 8) reinterpret_cast<uint32_t*>(out + 2 * it)[rank] = c;
+      const unsigned eighth = __ballot_sync(kFull, ((fresh >> lane) & 1u) && rank == 7);
+      ++it, pos += __ffs(eighth);
+      continue;
+    }
+    // More than 32 residues: one after the other (every lane the same).
+    int k = 0, d = pos;
+    uint32_t got[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (; d < have && k < 8; ++d) {
+      const uint32_t v = buf[d];
+      bool again = false;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) again |= (j < k) & (got[j] == v);
+      if (!again) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-          if (j == k) idx[j] = c;
+          if (j == k) got[j] = v;
         ++k;
       }
     }
-    uint4* o4 = reinterpret_cast<uint4*>(out + 8 * it);
-    o4[0] = make_uint4(idx[0], idx[1], idx[2], idx[3]);
-    o4[1] = make_uint4(idx[4], idx[5], idx[6], idx[7]);
+    more = k < 8;  // ran out of residues: this sample begins again with more
+    if (!more) {
+      if (lane == 0) {
+        out[2 * it] = make_uint4(got[0], got[1], got[2], got[3]);
+        out[2 * it + 1] = make_uint4(got[4], got[5], got[6], got[7]);
+      }
+      ++it, pos = d;
+    }
   }
 }
 
@@ -171,8 +271,10 @@ __device__ void jacobi3(double (&A)[3][3], double (&V)[3][3]) {
       for (int q = p + 1; q < 3; ++q) {
         if (A[p][q] == 0.0) continue;
         const double theta = (A[q][q] - A[p][p]) / (2.0 * A[p][q]);
-        const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-        const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
+        // (IEEE reciprocals: five FP64 operations where a division is nine)
+        const double rt = __drcp_rn(fabs(theta) + sqrt(theta * theta + 1.0));
+        const double t = theta >= 0.0 ? rt : -rt;
+        const double c = __drcp_rn(sqrt(t * t + 1.0)), sn = t * c;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           const double akp = A[k][p], akq = A[k][q];
@@ -310,9 +412,22 @@ __device__ bool ep_finish(const double* fm, const double* ta, const double* tb, 
   for (int i = 0; i < 9; ++i) nrm += full[i] * full[i];
   nrm = sqrt(nrm);
   if (!(nrm > 1e-15)) return false;
+  const double rn = __drcp_rn(nrm);
 #pragma unroll
-  for (int i = 0; i < 9; ++i) F[i] = full[i] / nrm;
+  for (int i = 0; i < 9; ++i) F[i] = quotient_by(full[i], nrm, rn);
   return true;
+}
+
+// |x| rounded to FP32, as an integer in the same order (-1 for NaN): the FP64
+// pipe, the bound of the fit, also executes the hardware's conversion.
+__device__ __forceinline__ int magnitude_f32(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+  if (hi - (898u << 20) < (252u << 20)) {  // well inside FP32's normal range
+    const uint64_t b = ((uint64_t)(hi - (896u << 20)) << 32) | (uint32_t)__double2loint(x);
+    return (int)((b + 0x0fffffffull + ((b >> 29) & 1)) >> 29);  // to nearest, ties to even
+  }
+  const float f = fabsf((float)x);
+  return f == f ? __float_as_int(f) : -1;
 }
 
 // The 8-point hypothesis (geometry.rs:186-230 on eight correspondences).
@@ -342,14 +457,14 @@ __device__ bool ep_fundamental8(const double* uv, const uint32_t* idx, double* A
 #pragma unroll
   for (int c = 0; c < 9; ++c) perm |= (uint64_t)c << (4 * c);
   int rank = 8;
+  double rpiv = 0.0;
   for (int k = 0; k < 8; ++k) {
     // Pivot choice on FP32 magnitudes (the choice only steers stability);
     // a zero pivot is tested exactly.
-    int pr = k, pc = k;
-    float best = -1.0f;
+    int pr = k, pc = k, best = -1;
     for (int r = k; r < 8; ++r)
       for (int c = k; c < 9; ++c) {
-        const float v = fabsf((float)AS(r, c));
+        const int v = magnitude_f32(AS(r, c));
         if (v > best) best = v, pr = r, pc = c;
       }
     if (AS(pr, pc) == 0.0) {
@@ -357,7 +472,7 @@ __device__ bool ep_fundamental8(const double* uv, const uint32_t* idx, double* A
       break;
     }
     if (pr != k)
-      for (int c = 0; c < 9; ++c) {
+      for (int c = k; c < 9; ++c) {
         const double t = AS(k, c);
         AS(k, c) = AS(pr, c), AS(pr, c) = t;
       }
@@ -370,11 +485,12 @@ __device__ bool ep_fundamental8(const double* uv, const uint32_t* idx, double* A
       perm &= ~((uint64_t)15 << (4 * k)) & ~((uint64_t)15 << (4 * pc));
       perm |= (b << (4 * k)) | (a << (4 * pc));
     }
-    const double rpiv = 1.0 / AS(k, k);
+    rpiv = __drcp_rn(AS(k, k));
     for (int r = k + 1; r < 8; ++r) {
       const double m = AS(r, k) * rpiv;
       for (int c = k + 1; c < 9; ++c) AS(r, c) -= m * AS(k, c);
     }
+    if (k < 7) AS(k + 1, k) = rpiv;  // kept for the back-substitution
   }
   // Null vector: the free (last unpivoted) unknown is 1, the rest follow by
   // back-substitution through the upper-triangular rows 0..rank-1.
@@ -384,7 +500,7 @@ __device__ bool ep_fundamental8(const double* uv, const uint32_t* idx, double* A
   for (int k = rank - 1; k >= 0; --k) {
     double acc = 0.0;
     for (int c = k + 1; c < 9; ++c) acc += AS(k, c) * (c == rank ? 1.0 : (c < rank ? x[c] : 0.0));
-    x[k] = -acc / AS(k, k);
+    x[k] = quotient_by(-acc, AS(k, k), k < 7 ? AS(k + 1, k) : rpiv);
   }
 #undef AS
   double fm[9];
@@ -400,8 +516,9 @@ __device__ bool ep_fundamental8(const double* uv, const uint32_t* idx, double* A
 #pragma unroll
   for (int c = 0; c < 9; ++c) nn += fm[c] * fm[c];
   nn = sqrt(nn);
+  const double rnn = __drcp_rn(nn);
 #pragma unroll
-  for (int c = 0; c < 9; ++c) fm[c] /= nn;
+  for (int c = 0; c < 9; ++c) fm[c] = quotient_by(fm[c], nn, rnn);
   return ep_finish(fm, ta, tb, F);
 }
 
@@ -420,6 +537,10 @@ __global__ void __launch_bounds__(kFitThreads) ransac_fit_kernel(RansacArgs A) {
   if (!ep_fundamental8(A.uv + 4 * (size_t)b, idx, As + threadIdx.x, kFitThreads, F)) return;
 #pragma unroll
   for (int j = 0; j < 9; ++j) A.F[9 * h + j] = F[j];
+  float4* f = A.F32 + 3 * h;
+  f[0] = make_float4((float)F[0], (float)F[1], (float)F[2], (float)F[3]);
+  f[1] = make_float4((float)F[4], (float)F[5], (float)F[6], (float)F[7]);
+  f[2] = make_float4((float)F[8], 0.0f, 0.0f, 0.0f);
   A.valid[h] = 1;
 }
 
@@ -475,7 +596,7 @@ __device__ __forceinline__ int inlier_fp32(const Hyp32& H, float4 c, float t2) {
   return -1;
 }
 
-constexpr int kCountTile = 1024;
+constexpr int kCountTile = 2048;
 
 // First-tier bounds of one hypothesis over one tile of correspondences, from
 // the tile's largest coordinate magnitudes (ax, ay, bx, by): every |f_k| is
@@ -504,9 +625,10 @@ __device__ __forceinline__ TileBound tile_bound(const Hyp32& H, float4 m) {
   return B;
 }
 
-// 1 / 0 surely in / out by the tile's constant bounds, -1 undecided.
-__device__ __forceinline__ int inlier_tile(const Hyp32& H, const TileBound& B, float4 c,
-                                           float t2) {
+// Whether surely in / surely out by the tile's constant bounds (neither:
+// undecided).
+__device__ __forceinline__ void inlier_tile(const Hyp32& H, const TileBound& B, float4 c, float t2,
+                                            bool& in, bool& out) {
   constexpr float u = 5.9604645e-8f;
   const float* f = H.f;
   const float f0 = fmaf(f[0], c.x, fmaf(f[1], c.y, f[2]));
@@ -518,52 +640,49 @@ __device__ __forceinline__ int inlier_tile(const Hyp32& H, const TileBound& B, f
   const float d = fmaf(f0, f0, fmaf(f1, f1, fmaf(g0, g0, g1 * g1)));
   const float dd = fmaf(8.0f * u, d, B.dd);
   const float lo = d - dd;
-  if (lo > 2e-18f) {
-    const float a = ae + B.de;
-    if (a * a < t2 * lo * (1.0f - 32.0f * u)) return 1;
-    const float o = ae - B.de;
-    if (o > 0.0f && o * o > t2 * (d + dd) * (1.0f + 32.0f * u)) return 0;
-  }
-  return -1;
+  const float a = ae + B.de, o = ae - B.de;
+  const bool clear = lo > 2e-18f;
+  in = clear && a * a < t2 * lo * (1.0f - 32.0f * u);
+  out = clear && o > 0.0f && o * o > t2 * (d + dd) * (1.0f + 32.0f * u);
 }
 
-// CTA per (pair, 32 hypotheses); each warp tests four hypotheses against
-// every correspondence of the pair, the pair's FP32 coordinates staged
-// through shared memory a tile at a time.  Tests are decided by the tile's
-// constant bounds, else by the correspondence's own bounds, else in FP64.
+// Inlier counts: a warp per hypothesis at a time, over the pair's FP32
+// coordinates in shared memory (a tile of them at a time where they are
+// more).  Tests are decided by the tile's constant bounds, else by the
+// correspondence's own bounds, else in FP64.
+//
+// Only the first hypothesis with the most inliers is wanted: one that could
+// not reach the CTA's best count any more, were all its remaining tests
+// inliers, is left with a count of 0 (a sample with one mismatch in it, nine
+// of ten at a quarter of mismatches, is through after some third of the
+// tests).  gridDim.x / pairs CTAs share a pair, a bound each.  Four tests a
+// lane are in flight, and both outcomes of a test are formed without a
+// branch.  1603 pairs x 600 x 1300 tests: 3.9 ms with every test made, four
+// hypotheses a warp.
 __global__ void __launch_bounds__(kCountThreads) ransac_count_kernel(RansacArgs A,
-                                                                     const float4* uv32) {
+                                                                     const float4* uv32,
+                                                                     int parts) {
   __shared__ float4 tile[kCountTile];
   __shared__ float4 wmax[kCountThreads / 32];
-  const int blocks_per_pair = (A.iters + kHypPerCountCta - 1) / kHypPerCountCta;
-  const int64_t q = blockIdx.x / blocks_per_pair;
-  const int hb = (int)(blockIdx.x % blocks_per_pair) * kHypPerCountCta;
+  __shared__ int best;
+  constexpr int kWarps = kCountThreads / 32, kTests = 4;
+  const int64_t q = blockIdx.x / parts;
+  const int part = (int)(blockIdx.x % parts);
   const int64_t p = A.p0 + q;
   const uint32_t b = A.match_ptr[p], n = A.match_ptr[p + 1] - b;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kPerWarp = kHypPerCountCta / (kCountThreads / 32);
   const float t2 = (float)A.t2;
-  Hyp32 H[kPerWarp];
-  bool ok[kPerWarp];
-  int cnt[kPerWarp];
-#pragma unroll
-  for (int j = 0; j < kPerWarp; ++j) {
-    const int it = hb + warp * kPerWarp + j;
-    const int64_t h = q * A.iters + it;
-    ok[j] = n >= 12 && it < A.iters && A.valid[h];
-    cnt[j] = 0;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) H[j].f[k] = ok[j] ? (float)A.F[9 * h + k] : 0.0f;
-  }
+  const int h0 = (int)((int64_t)A.iters * part / parts),
+            h1 = (int)((int64_t)A.iters * (part + 1) / parts);
   if (n < 12) {
-    if (lane < kPerWarp && hb + warp * kPerWarp + lane < A.iters)
-      A.count[q * A.iters + hb + warp * kPerWarp + lane] = 0;
+    for (int it = h0 + threadIdx.x; it < h1; it += kCountThreads) A.count[q * A.iters + it] = 0;
     return;
   }
-  for (uint32_t t0 = 0; t0 < n; t0 += kCountTile) {
-    const uint32_t tn = min((uint32_t)kCountTile, n - t0);
+  if (threadIdx.x == 0) best = 0;
+  float4 m;
+  auto load_tile = [&](uint32_t t0, uint32_t tn) {
     __syncthreads();
-    float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+    m = make_float4(0.f, 0.f, 0.f, 0.f);
     for (uint32_t i = threadIdx.x; i < tn; i += kCountThreads) {
       const float4 c = uv32[b + t0 + i];
       tile[i] = c;
@@ -580,36 +699,70 @@ __global__ void __launch_bounds__(kCountThreads) ransac_count_kernel(RansacArgs 
     if (lane == 0) wmax[warp] = m;
     __syncthreads();
 #pragma unroll
-    for (int w = 0; w < kCountThreads / 32; ++w) {
+    for (int w = 0; w < kWarps; ++w) {
       const float4 v = wmax[w];
       m.x = fmaxf(m.x, v.x), m.y = fmaxf(m.y, v.y), m.z = fmaxf(m.z, v.z), m.w = fmaxf(m.w, v.w);
     }
-    TileBound TB[kPerWarp];
+  };
+  const bool one_tile = n <= (uint32_t)kCountTile;
+  if (one_tile) load_tile(0, n);
+  // Every warp makes the same number of rounds (a tile is loaded by all).
+  for (int hb = h0; hb < h1; hb += kWarps) {
+    const int it = hb + warp;
+    const int64_t h = q * A.iters + it;
+    bool live = it < h1 && A.valid[h];
+    Hyp32 H;
+    {
+      const float4* f = A.F32 + 3 * h;
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 a = live ? f[0] : z, c = live ? f[1] : z, e = live ? f[2] : z;
+      H.f[0] = a.x, H.f[1] = a.y, H.f[2] = a.z, H.f[3] = a.w;
+      H.f[4] = c.x, H.f[5] = c.y, H.f[6] = c.z, H.f[7] = c.w, H.f[8] = e.x;
+    }
+    int cnt = 0;
+    for (uint32_t t0 = 0; t0 < n; t0 += kCountTile) {
+      const uint32_t tn = min((uint32_t)kCountTile, n - t0);
+      if (!one_tile) load_tile(t0, tn);
+      if (!live) continue;
+      const TileBound TB = tile_bound(H, m);
+      for (uint32_t i0 = 0; i0 < tn; i0 += 32 * kTests) {
+        bool in[kTests], out[kTests];
 #pragma unroll
-    for (int j = 0; j < kPerWarp; ++j) TB[j] = tile_bound(H[j], m);
-    for (uint32_t i = lane; i < tn; i += 32) {
-      const float4 c = tile[i];
-#pragma unroll
-      for (int j = 0; j < kPerWarp; ++j) {
-        if (!ok[j]) continue;
-        int r = inlier_tile(H[j], TB[j], c, t2);
-        if (r < 0) r = inlier_fp32(H[j], c, t2);
-        if (r < 0) {
-          const int64_t h = q * A.iters + hb + warp * kPerWarp + j;
-          const double* u64 = A.uv + 4 * ((size_t)b + t0 + i);
-          r = ep_sampson(A.F + 9 * h, u64[0], u64[1], u64[2], u64[3]) < A.t2;
+        for (int j = 0; j < kTests; ++j) {
+          const uint32_t i = i0 + 32 * j + lane;
+          inlier_tile(H, TB, tile[i < tn ? i : 0], t2, in[j], out[j]);
+          in[j] = in[j] && i < tn, out[j] = out[j] || i >= tn;
         }
-        cnt[j] += r;
+#pragma unroll
+        for (int j = 0; j < kTests; ++j) {
+          if (__any_sync(kFull, !in[j] && !out[j])) {
+            if (!in[j] && !out[j]) {
+              const uint32_t i = i0 + 32 * j + lane;
+              int r = inlier_fp32(H, tile[i], t2);
+              if (r < 0) {
+                const double* u64 = A.uv + 4 * ((size_t)b + t0 + i);
+                r = ep_sampson(A.F + 9 * h, u64[0], u64[1], u64[2], u64[3]) < A.t2;
+              }
+              in[j] = r != 0;
+            }
+            __syncwarp();
+          }
+          cnt += __popc(__ballot_sync(kFull, in[j]));
+        }
+        // strictly less: of equal counts the first hypothesis wins
+        const int64_t left = (int64_t)n - t0 - i0 - 32 * kTests;
+        if (left > 0 && cnt + left < *(volatile int*)&best) {
+          live = false;
+          cnt = 0;
+          break;
+        }
       }
     }
-  }
-#pragma unroll
-  for (int j = 0; j < kPerWarp; ++j) {
-    int v = cnt[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    const int it = hb + warp * kPerWarp + j;
-    if (lane == 0 && it < A.iters) A.count[q * A.iters + it] = ok[j] ? v : 0;
+    if (it < h1 && lane == 0) {
+      A.count[h] = cnt;
+      if (live) atomicMax(&best, cnt);
+    }
+    __syncwarp();
   }
 }
 
@@ -727,11 +880,12 @@ __global__ void __launch_bounds__(kRefitThreads) ransac_select_kernel(RansacArgs
   if (threadIdx.x == 0) A.best[p] = hbest, A.n_inl[p] = nb;
   if (nb < 8) return;
   // normalise (geometry.rs:161-183) of both sides over the inliers.
-  const double nn = (double)nb;
+  const double nn = (double)nb, rnn = __drcp_rn(nn);
   double sa = 0.0, sb = 0.0, sc = 0.0, sd = 0.0;
   for (int i = threadIdx.x; i < nb; i += kRefitThreads) {
     const double* u = U + 4 * (size_t)list[i];
-    sa += u[0] / nn, sb += u[1] / nn, sc += u[2] / nn, sd += u[3] / nn;
+    sa += quotient_by(u[0], nn, rnn), sb += quotient_by(u[1], nn, rnn);
+    sc += quotient_by(u[2], nn, rnn), sd += quotient_by(u[3], nn, rnn);
   }
   const double max_ = cta_sum_d(sa, dred), may = cta_sum_d(sb, dred);
   const double mbx = cta_sum_d(sc, dred), mby = cta_sum_d(sd, dred);
@@ -793,11 +947,12 @@ __global__ void __launch_bounds__(kRefitThreads) ransac_select_kernel(RansacArgs
   int cnt = 0;
   for (uint32_t i = threadIdx.x; i < n; i += kRefitThreads) {
     const double* u = U + 4 * (size_t)i;
-    cnt += ep_sampson(Fs, u[0], u[1], u[2], u[3]) < A.t2;
+    list[i] = ep_sampson(Fs, u[0], u[1], u[2], u[3]) < A.t2;  // (the index list is done with)
+    cnt += list[i];
   }
   const int nr = cta_sum_int(cnt, wsum);
   if (nr < nb) return;
-  mark_inliers(Fs, U, n, A.t2, flag, list, wsum);
+  for (uint32_t i = threadIdx.x; i < n; i += kRefitThreads) flag[i] = (uint8_t)list[i];
   if (threadIdx.x == 0) A.n_inl[p] = nr, A.refit[p] = 1;
 }
 
@@ -950,6 +1105,29 @@ struct PairsIn {
   }
 };
 
+// A second stream for a call's large copy, and an event for the order.
+struct CopySide {
+  cudaStream_t s = nullptr;
+  cudaEvent_t e = nullptr;
+  // From here on (buffers made, the caller's earlier work done).
+  void fork(cudaStream_t main) {
+    check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "copy stream");
+    check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+    check(cudaEventRecord(e, main), "fork");
+    check(cudaStreamWaitEvent(s, e, 0), "fork");
+  }
+  // `main` waits for the copies so far.
+  void join(cudaStream_t main) {
+    if (!s) return;
+    check(cudaEventRecord(e, s), "join");
+    check(cudaStreamWaitEvent(main, e, 0), "join");
+  }
+  ~CopySide() {
+    if (s) cudaStreamSynchronize(s), cudaStreamDestroy(s);
+    if (e) cudaEventDestroy(e);
+  }
+};
+
 }  // namespace
 }  // namespace ba
 
@@ -964,8 +1142,14 @@ extern "C" ba_status ba_ransac_fundamental(const ba_pair_matches* m, double thre
     if (iters < 0 || iters > (1 << 20)) throw BadInput("iters must be in 0..2^20");
     cudaStream_t s = (cudaStream_t)stream;
     PairsIn P;
-    P.load(m, m && !m->seed, (int64_t)1 << 32, nullptr, 0, s);
+    P.load(m, m && !m->seed, (int64_t)1 << 32, nullptr, 0, s, false);
     const int64_t np = P.np, nm = P.nm;
+    // A large call's correspondences are copied while the samples are drawn.
+    CopySide side;
+    if (nm > (int64_t(1) << 18)) side.fork(s);
+    if (nm > 0)
+      check(cudaMemcpyAsync(P.uv.p, m->uv, 32 * nm, cudaMemcpyDefault, side.s ? side.s : s),
+            "copy in");
     DevBuf<uint64_t> seed;
     if (m->seed) {
       upload_n(seed, m->seed, np, s);
@@ -981,19 +1165,34 @@ extern "C" ba_status ba_ransac_fundamental(const ba_pair_matches* m, double thre
     const int64_t ch = std::max<int64_t>(cp * iters, 1);
     DevBuf<uint32_t> samples(8 * ch, s);
     DevBuf<double> F(9 * ch, s);
+    DevBuf<float4> F32(3 * ch, s);
     DevBuf<uint8_t> valid(ch, s);
     DevBuf<int32_t> count(ch, s);
     DevBuf<float4> uv32(std::max<int64_t>(nm, 1), s);
-    if (nm > 0) BA_LAUNCH(uv_f32_kernel<<<grid_for(nm, 256), 256, 0, s>>>(nm, P.uv, uv32));
+    // Counting: two CTAs a pair (1603 pairs of unequal size: 2.25 ms; one 2.45,
+    // three 2.28), more where that leaves SMs with fewer than four, but at
+    // least eight hypotheses a warp, so that the bound of a CTA's first counts
+    // serves most of its hypotheses.
+    int dev = 0, n_sm = 0;
+    check(cudaGetDevice(&dev), "cudaGetDevice");
+    check(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev), "attribute");
+    auto join_copy = [&] {
+      side.join(s);
+      if (nm > 0) BA_LAUNCH(uv_f32_kernel<<<grid_for(nm, 256), 256, 0, s>>>(nm, P.uv, uv32));
+    };
+    if (np == 0 || iters == 0) join_copy();
     for (int64_t p0 = 0; p0 < np; p0 += cp) {
       const int64_t n = std::min(cp, np - p0);
-      RansacArgs A{p0, n, P.match_ptr, P.uv, seed, iters, thresh_px * thresh_px, samples, F,
+      RansacArgs A{p0, n, P.match_ptr, P.uv, seed, iters, thresh_px * thresh_px, samples, F, F32,
                    valid, count, scratch, d_inl, d_n, d_best, d_refit, P.err};
       if (iters > 0) {
-        BA_LAUNCH(ransac_sample_kernel<<<grid_for(n, 128), 128, 0, s>>>(A));
+        BA_LAUNCH(ransac_sample_kernel<<<(unsigned)n, 32, 0, s>>>(A, draw_jump()));
+        if (p0 == 0) join_copy();
         BA_LAUNCH(ransac_fit_kernel<<<grid_for(n * iters, kFitThreads), kFitThreads, 0, s>>>(A));
-        const int64_t bpp = (iters + kHypPerCountCta - 1) / kHypPerCountCta;
-        BA_LAUNCH(ransac_count_kernel<<<(unsigned)(n * bpp), kCountThreads, 0, s>>>(A, uv32));
+        const int64_t most = std::max<int64_t>(1, iters / (8 * (kCountThreads / 32)));
+        const int parts = (int)std::min<int64_t>(most, std::max<int64_t>(2, 4 * n_sm / n));
+        BA_LAUNCH(ransac_count_kernel<<<(unsigned)(n * parts), kCountThreads, 0, s>>>(A, uv32,
+                                                                                     parts));
       }
       BA_LAUNCH(ransac_select_kernel<<<(unsigned)n, kRefitThreads, 0, s>>>(A));
     }
@@ -1034,20 +1233,8 @@ extern "C" ba_status ba_pair_fits(const ba_pair_matches* m, const double* rot, c
     for (int64_t p = 0; p < np; ++p) most = std::max(most, ptr[p + 1] - ptr[p]);
     DevBuf<uint64_t> key(most > kFitKeys ? nm : 1, s);
     FitsArgs A{0, P.pair_cam, P.match_ptr, P.uv, d_rot, d_center, d_intr, d_group, key, med};
-    struct Side {
-      cudaStream_t s = nullptr;
-      cudaEvent_t e = nullptr;
-      ~Side() {
-        if (s) cudaStreamSynchronize(s), cudaStreamDestroy(s);
-        if (e) cudaEventDestroy(e);
-      }
-    } side;
-    if (nm > (int64_t(1) << 20)) {
-      check(cudaStreamCreateWithFlags(&side.s, cudaStreamNonBlocking), "copy stream");
-      check(cudaEventCreateWithFlags(&side.e, cudaEventDisableTiming), "event");
-      check(cudaEventRecord(side.e, s), "fork");  // the buffer exists, the caller's work is done
-      check(cudaStreamWaitEvent(side.s, side.e, 0), "fork");
-    }
+    CopySide side;
+    if (nm > (int64_t(1) << 20)) side.fork(s);
     for (int64_t p0 = 0; p0 < np;) {
       int64_t p1 = np;
       if (side.s && p0 == 0) {
@@ -1059,10 +1246,7 @@ extern "C" ba_status ba_pair_fits(const ba_pair_matches* m, const double* rot, c
         check(cudaMemcpyAsync(P.uv.p + 4 * b, m->uv + 4 * b, 32 * n, cudaMemcpyDefault,
                               side.s ? side.s : s),
               "copy in");
-      if (side.s) {
-        check(cudaEventRecord(side.e, side.s), "piece");
-        check(cudaStreamWaitEvent(s, side.e, 0), "piece");
-      }
+      side.join(s);
       A.p0 = p0;
       BA_LAUNCH(pair_fits_kernel<<<(unsigned)(p1 - p0), kFitsThreads, 0, s>>>(A));
       p0 = p1;
