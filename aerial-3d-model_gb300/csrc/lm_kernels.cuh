@@ -13,6 +13,9 @@ constexpr int kLinW = 28;  // per-observation record: jc 12, jp 6, jg 6, e 2, w,
 
 enum { LOSS_CAUCHY = 0, LOSS_HUBER = 1 };
 
+// Values from one lens entry's factor to the next's: 9, on 16-byte boundaries.
+constexpr int kZlPitch = 12;
+
 template <typename R>
 struct IterBufs {
   R* lin;      // [no][kLinW]
@@ -21,7 +24,7 @@ struct IterBufs {
   // Jg^T r' (3) with r' = w (e - Jp V^-1 v), computed from FP64 values.
   R* gsub;
   R* Z;        // [no][18]: Y_k L (L L^T = V^-1)
-  R* Zl;       // [nl][9]: lens entry, top 3x3
+  R* Zl;       // [nl][kZlPitch]: lens entry, top 3x3 (9)
   double* ptL;   // [np][6]: l00 l10 l11 l20 l21 l22
   double* ptzv;  // [np][3]: L^T v
   uint8_t* kept;  // [np]: 0 skipped, 1 kept, 2 kept and ill-conditioned (mixed form)
@@ -202,7 +205,7 @@ __device__ __forceinline__ void point_system(const Prob& P, const StateView& st,
       for (int i = 0; i < 9; ++i) B.gsub[(size_t)k * 9 + i] = (R)0;
     }
     for (uint32_t j = S.lens_ptr[p]; j < S.lens_ptr[p + 1]; ++j)
-      for (int i = 0; i < 9; ++i) B.Zl[(size_t)j * 9 + i] = (R)0;
+      for (int i = 0; i < 9; ++i) B.Zl[(size_t)j * kZlPitch + i] = (R)0;
     return;
   }
   // V, v and the Y / Z products accumulate in the storage precision R; the 3x3
@@ -297,7 +300,7 @@ __device__ __forceinline__ void point_system(const Prob& P, const StateView& st,
         Y[3 * a + 2] += (ga * j2 + gb * j5) * w;
       }
     }
-    R* Zl = B.Zl + (size_t)j * 9;
+    R* Zl = B.Zl + (size_t)j * kZlPitch;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const R y0 = Y[3 * a], y1 = Y[3 * a + 1], y2 = Y[3 * a + 2];
@@ -573,7 +576,7 @@ static __device__ __noinline__ void point_system_mixed_ill(const Prob& P, const 
       for (int i = 0; i < 9; ++i) B.gsub[(size_t)k * 9 + i] = 0.0f;
     }
     for (uint32_t j = S.lens_ptr[p]; j < S.lens_ptr[p + 1]; ++j)
-      for (int i = 0; i < 9; ++i) B.Zl[(size_t)j * 9 + i] = 0.0f;
+      for (int i = 0; i < 9; ++i) B.Zl[(size_t)j * kZlPitch + i] = 0.0f;
     return;
   }
   const double zv0 = L[0] * v[0] + L[1] * v[1] + L[3] * v[2];
@@ -639,7 +642,7 @@ static __device__ __noinline__ void point_system_mixed_ill(const Prob& P, const 
         Y[3 * a + 2] += (ga * j2 + gb * j5) * w;
       }
     }
-    float* Zl = B.Zl + (size_t)j * 9;
+    float* Zl = B.Zl + (size_t)j * kZlPitch;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const double y0 = Y[3 * a], y1 = Y[3 * a + 1], y2 = Y[3 * a + 2];
@@ -779,7 +782,7 @@ __device__ __forceinline__ void point_mixed_finish(
   if (!sum) {  // fewer than two observations (ba.rs:238)
     B.kept[p] = 0;
     for (uint32_t j = l0; j < l1; ++j)
-      for (int i = 0; i < 9; ++i) B.Zl[(size_t)j * 9 + i] = 0.0f;
+      for (int i = 0; i < 9; ++i) B.Zl[(size_t)j * kZlPitch + i] = 0.0f;
     return;
   }
   double V[6], v[3];
@@ -862,7 +865,7 @@ __device__ __forceinline__ void point_mixed_finish(
         Y[3 * a + 2] += (ga * j2 + gb * j5) * w;
       }
     }
-    float* Zl = B.Zl + (size_t)j * 9;
+    float* Zl = B.Zl + (size_t)j * kZlPitch;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const float y0 = Y[3 * a], y1 = Y[3 * a + 1], y2 = Y[3 * a + 2];
@@ -1827,35 +1830,79 @@ __device__ __forceinline__ void load_Z24(const float* s, float* z) {
 __device__ __forceinline__ void load_Z24(const double*, double*) {}  // FP32 layout only
 
 template <typename R>
-__device__ __forceinline__ void load_Z(const IterBufs<R>& B, int64_t no, uint32_t eid, R* z) {
-  if ((int64_t)eid < no) {
-    if (sizeof(R) == 4 && B.zpitch == 24)
-      load_Z24(B.Z + (size_t)eid * 24, z);
-    else
-      load_Z18(B.Z + (size_t)eid * B.zpitch, z);
+__device__ __forceinline__ void load_Z(const IterBufs<R>& B, uint32_t k, R* z) {
+  if (sizeof(R) == 4 && B.zpitch == 24)
+    load_Z24(B.Z + (size_t)k * 24, z);
+  else
+    load_Z18(B.Z + (size_t)k * B.zpitch, z);
+}
+// A lens entry's nine values.
+__device__ __forceinline__ void load_Zl(const double* s, double* z) {
+  const double2* v = reinterpret_cast<const double2*>(s);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double2 t = __ldg(v + i);
+    z[2 * i] = t.x, z[2 * i + 1] = t.y;
+  }
+  z[8] = __ldg(s + 8);
+}
+__device__ __forceinline__ void load_Zl(const float* s, float* z) {
+  const float4* v = reinterpret_cast<const float4*>(s);
+  const float4 a = __ldg(v), b = __ldg(v + 1);
+  z[0] = a.x, z[1] = a.y, z[2] = a.z, z[3] = a.w;
+  z[4] = b.x, z[5] = b.y, z[6] = b.z, z[7] = b.w;
+  z[8] = __ldg(s + 8);
+}
+
+// What the pairs of a destination block are, and so which of its 36 entries
+// their products Z_a Z_b^T reach: a lens entry has three rows (the products
+// with its missing ones are zero), and an entry with itself gives a symmetric
+// product, whose two halves are the same operations.
+enum class SchurKind { kFull, kCamera, kCameraLens, kLens, kLenses };
+
+template <SchurKind K>
+struct SchurOut {
+  static constexpr int kRows = K == SchurKind::kLens || K == SchurKind::kLenses ? 3 : 6;
+  static constexpr int kCols = K == SchurKind::kFull || K == SchurKind::kCamera ? 6 : 3;
+  static constexpr bool kSym = K == SchurKind::kCamera || K == SchurKind::kLens;
+  static constexpr int kN = kSym ? kRows * (kRows + 1) / 2 : kRows * kCols;
+};
+
+// Warp sum of N values per lane by halving: after the offsets 16, 8, 4, 2, 1
+// the lane holds the totals of values off .. off + cnt - 1 in out[].
+template <int O, int N, int M, typename R>
+__device__ __forceinline__ void warp_halve(const R (&v)[N], int lane, int& off, int& cnt,
+                                           R (&out)[M]) {
+  if constexpr (O == 0) {
+    static_assert(N <= M, "results per lane");
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = v[i];
   } else {
-    const R* s = B.Zl + (size_t)(eid - no) * 9;
+    constexpr int H = (N + 1) / 2;
+    const bool up = lane & O;
+    R w[H];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) z[i] = s[i];
-#pragma unroll
-    for (int i = 9; i < 18; ++i) z[i] = (R)0;
+    for (int i = 0; i < H; ++i) {
+      const int j = H + i < N ? H + i : i;  // (odd N: an upper lane's last one is not used)
+      const R recv = __shfl_xor_sync(kFull, up ? v[i] : v[j], O);
+      w[i] = (up ? v[j] : v[i]) + recv;
+    }
+    off += up ? H : 0;
+    cnt = up ? cnt - H : min(cnt, H);
+    warp_halve<O / 2>(w, lane, off, cnt, out);
   }
 }
 
-template <typename R>
-// FP32 form: 3 CTAs per SM (80 registers; the kernel is bound by the latency
-// of its gathers, and the extra resident warps hide more of it).
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 1)
-    schur_kernel(Prob P, StructView S, IterBufs<R> B, const int32_t* active) {
-  const int64_t sub = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// The sum over pairs [b, e) of a destination block into part[36].
+template <SchurKind K, typename R>
+__device__ __forceinline__ void schur_segment(const Prob& P, const StructView& S,
+                                              const IterBufs<R>& B, uint32_t b, uint32_t e,
+                                              double* part) {
+  using O = SchurOut<K>;
   const int lane = threadIdx.x & 31;
-  if (sub >= S.nsub) return;
-  const uint32_t slot = S.sub_slot[sub];
-  if (!active[P.blk_model[S.slot_row[slot]]]) return;
-  R acc[36];
+  R acc[O::kN];
 #pragma unroll
-  for (int i = 0; i < 36; ++i) acc[i] = (R)0;
-  const uint32_t b = S.sub_begin[sub], e = S.sub_end[sub];
+  for (int i = 0; i < O::kN; ++i) acc[i] = (R)0;
   // The next pair's entry is loaded while this pair's factors are gathered
   // and multiplied (one dependent load less per pair on the critical path).
   uint64_t nxt = b + lane < e ? S.pairs[b + lane] : kSentinel;
@@ -1863,49 +1910,92 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 1)
     const uint64_t pr = nxt;
     nxt = i + 32 < e ? S.pairs[i + 32] : kSentinel;
     if (pr == kSentinel) continue;
-    if ((int64_t)(pr & 0xffffffffu) >= P.no + S.nl || (int64_t)(pr >> 32) >= P.no + S.nl) continue;
-    R za[18], zb[18];
-    load_Z(B, P.no, (uint32_t)(pr & 0xffffffffu), za);
-    load_Z(B, P.no, (uint32_t)(pr >> 32), zb);
+    const uint32_t ea = (uint32_t)pr, eb = (uint32_t)(pr >> 32);
+    if ((int64_t)ea >= P.no + S.nl || (int64_t)eb >= P.no + S.nl) continue;
+    R za[3 * O::kRows], zb[3 * O::kCols];
+    if constexpr (O::kRows == 6)
+      load_Z(B, ea, za);
+    else
+      load_Zl(B.Zl + (size_t)(ea - P.no) * kZlPitch, za);
+    if constexpr (O::kSym) {
 #pragma unroll
-    for (int r = 0; r < 6; ++r)
-#pragma unroll
-      for (int c = 0; c < 6; ++c)
-        acc[6 * r + c] += za[3 * r] * zb[3 * c] + za[3 * r + 1] * zb[3 * c + 1] +
-                          za[3 * r + 2] * zb[3 * c + 2];
-  }
-  // Warp sum of the 36 entries, halving twice (36 -> 18 -> 9 values per lane)
-  // before a butterfly on the last 9: 54 adds per lane instead of 180 (the
-  // adds are FP64 warp instructions in the plain form).  Lanes 0, 8, 16, 24
-  // then hold entries 0-8, 9-17, 18-26, 27-35.
-  R a[18];
-  {
-    const bool up = lane & 16;
-#pragma unroll
-    for (int i = 0; i < 18; ++i) {
-      const R recv = __shfl_xor_sync(kFull, up ? acc[i] : acc[18 + i], 16);
-      a[i] = (up ? acc[18 + i] : acc[i]) + recv;
+      for (int t = 0; t < 3 * O::kRows; ++t) zb[t] = za[t];
+    } else if constexpr (O::kCols == 6) {
+      load_Z(B, eb, zb);
+    } else {
+      load_Zl(B.Zl + (size_t)(eb - P.no) * kZlPitch, zb);
     }
-  }
-  R v[9];
-  {
-    const bool up = lane & 8;
+    int n = 0;
 #pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      const R recv = __shfl_xor_sync(kFull, up ? a[i] : a[9 + i], 8);
-      v[i] = (up ? a[9 + i] : a[i]) + recv;
+    for (int r = 0; r < O::kRows; ++r)
+#pragma unroll
+      for (int c = O::kSym ? r : 0; c < O::kCols; ++c)
+        acc[n++] += za[3 * r] * zb[3 * c] + za[3 * r + 1] * zb[3 * c + 1] +
+                    za[3 * r + 2] * zb[3 * c + 2];
+  }
+  int off = 0, cnt = O::kN;
+  R v[2];
+  warp_halve<16>(acc, lane, off, cnt, v);
+  if constexpr (O::kN != 36) {
+    for (int i = lane; i < 36; i += 32)
+      if (i / 6 >= O::kRows || i % 6 >= O::kCols) part[i] = 0.0;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (i >= cnt) continue;
+    int r = 0, c = off + i;
+    if constexpr (O::kSym) {
+      for (int w = O::kRows; c >= w; c -= w, --w) ++r;
+      c += r;
+      part[6 * c + r] = (double)v[i];
+    } else {
+      r = c / O::kCols, c = c % O::kCols;
     }
+    part[6 * r + c] = (double)v[i];
   }
-#pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    v[i] += __shfl_xor_sync(kFull, v[i], 4);
-    v[i] += __shfl_xor_sync(kFull, v[i], 2);
-    v[i] += __shfl_xor_sync(kFull, v[i], 1);
-  }
-  if ((lane & 7) == 0) {
-    double* o = B.part + (size_t)sub * 36 + ((lane & 16) ? 18 : 0) + ((lane & 8) ? 9 : 0);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) o[i] = (double)v[i];
+}
+
+// Warp per sub-segment.  FP64 form: bound by its operations, of which the
+// kinds leave out what is zero or a mirror image (a sixth of them on the
+// 500-camera survey: 17 % of the pairs are an observation with itself, 20 % end
+// in a lens entry); 128 threads, three CTAs of 166 registers a thread.  FP32
+// form: bound by the latency of its gathers (three CTAs of 256 threads, 80
+// registers); an observation with itself is gathered once, a lens entry with
+// three loads.
+template <typename R>
+constexpr int kSchurThreads = sizeof(R) == 4 ? 256 : 128;
+
+template <typename R>
+__global__ void __launch_bounds__(kSchurThreads<R>, 3)
+    schur_kernel(Prob P, StructView S, IterBufs<R> B, const int32_t* active) {
+  const int64_t sub = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (sub >= S.nsub) return;
+  const uint32_t slot = S.sub_slot[sub];
+  const uint32_t row = S.slot_row[slot], col = S.slot_col[slot];
+  if (!active[P.blk_model[row]]) return;
+  const uint32_t b = S.sub_begin[sub], e = S.sub_end[sub];
+  double* part = B.part + (size_t)sub * 36;
+  if (P.blk_is_lens[row]) {  // its lens columns alone lie on or above the diagonal
+    if (row == col)
+      schur_segment<SchurKind::kLens>(P, S, B, b, e, part);
+    else
+      schur_segment<SchurKind::kLenses>(P, S, B, b, e, part);
+  } else if (P.blk_is_lens[col]) {
+    schur_segment<SchurKind::kCameraLens>(P, S, B, b, e, part);
+  } else if (row != col) {
+    schur_segment<SchurKind::kFull>(P, S, B, b, e, part);
+  } else {
+    // A point that a camera observes twice pairs two of the camera's entries.
+    bool same = true;
+    for (uint32_t i = b + lane; i < e; i += 32) {
+      const uint64_t pr = S.pairs[i];
+      same = same && (pr == kSentinel || (uint32_t)pr == (uint32_t)(pr >> 32));
+    }
+    if (__all_sync(kFull, same))
+      schur_segment<SchurKind::kCamera>(P, S, B, b, e, part);
+    else
+      schur_segment<SchurKind::kFull>(P, S, B, b, e, part);
   }
 }
 
@@ -2255,7 +2345,7 @@ __global__ void backsub_kernel(Prob P, StructView S, StateView cur, StateView tr
       }
     }
     for (uint32_t j = S.lens_ptr[p]; j < S.lens_ptr[p + 1]; ++j) {
-      const R* Z = B.Zl + (size_t)j * 9;
+      const R* Z = B.Zl + (size_t)j * kZlPitch;
       const R* d = B.x + 6 * (size_t)P.grp_blk[S.lens_grp[j]];
 #pragma unroll
       for (int r = 0; r < 3; ++r) {

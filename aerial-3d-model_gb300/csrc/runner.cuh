@@ -657,7 +657,7 @@ struct LmEngine {
       Z.release();
     else
       Z.alloc(at_least_1(no) * (z24 ? 24 : 18) + 4, s);
-    Zl.alloc(at_least_1(SB.nl) * 9, s);
+    Zl.alloc(at_least_1(SB.nl) * kZlPitch, s);
     ptL.alloc(at_least_1(np) * 6, s), ptzv.alloc(at_least_1(np) * 3, s);
     kept.alloc(at_least_1(np), s);
     camU.alloc(at_least_1(nc) * 21, s), camgj.alloc(at_least_1(nc) * 6, s);
@@ -1154,7 +1154,8 @@ struct LmEngine {
         set_sub_len(L);
         for (int rep = 0; rep < 3; ++rep) {
           check(cudaEventRecord(a, s), "event");
-          BA_LAUNCH(schur_kernel<R><<<grid_for(SB.nsub * 32, 256), 256, 0, s>>>(P, SV, B, active));
+          BA_LAUNCH(schur_kernel<R><<<grid_for(SB.nsub * 32, kSchurThreads<R>), kSchurThreads<R>, 0, s>>>(
+              P, SV, B, active));
           check(cudaEventRecord(b, s), "event");
           check(cudaEventSynchronize(b), "tune");
           float ms = 0;
@@ -1330,7 +1331,8 @@ struct LmEngine {
       return;
     }
     if (SB.nsub > 0)
-      BA_LAUNCH(schur_kernel<R><<<grid_for(SB.nsub * 32, 256), 256, 0, s>>>(P, SV, B, active));
+      BA_LAUNCH(schur_kernel<R><<<grid_for(SB.nsub * 32, kSchurThreads<R>), kSchurThreads<R>, 0, s>>>(
+              P, SV, B, active));
     if (n_fold > 0)
       BA_LAUNCH(schur_fold_kernel<<<n_fold, kFoldThreads, 0, s>>>(P, SV, part, fold_slots,
                                                                  active));
