@@ -13,8 +13,16 @@ constexpr int kLinW = 28;  // per-observation record: jc 12, jp 6, jg 6, e 2, w,
 
 enum { LOSS_CAUCHY = 0, LOSS_HUBER = 1 };
 
-// Values from one lens entry's factor to the next's: 9, on 16-byte boundaries.
-constexpr int kZlPitch = 12;
+// A lens entry's factor has nine values: eight in a record on a boundary of
+// its own size (two or four 16-byte loads), the ninth in an array behind the
+// records (IterBufs::Zl9).
+constexpr int kZlPitch = 8;
+
+// Value i of lens entry j.
+template <typename Bufs>
+__device__ __forceinline__ auto& zl_at(const Bufs& B, size_t j, int i) {
+  return i < kZlPitch ? B.Zl[j * kZlPitch + i] : B.Zl9[j];
+}
 
 template <typename R>
 struct IterBufs {
@@ -24,7 +32,8 @@ struct IterBufs {
   // Jg^T r' (3) with r' = w (e - Jp V^-1 v), computed from FP64 values.
   R* gsub;
   R* Z;        // [no][18]: Y_k L (L L^T = V^-1)
-  R* Zl;       // [nl][kZlPitch]: lens entry, top 3x3 (9)
+  R* Zl;       // [nl][kZlPitch]: lens entry, top 3x3, the first eight values
+  R* Zl9;      // [nl]: the ninth
   double* ptL;   // [np][6]: l00 l10 l11 l20 l21 l22
   double* ptzv;  // [np][3]: L^T v
   uint8_t* kept;  // [np]: 0 skipped, 1 kept, 2 kept and ill-conditioned (mixed form)
@@ -205,7 +214,7 @@ __device__ __forceinline__ void point_system(const Prob& P, const StateView& st,
       for (int i = 0; i < 9; ++i) B.gsub[(size_t)k * 9 + i] = (R)0;
     }
     for (uint32_t j = S.lens_ptr[p]; j < S.lens_ptr[p + 1]; ++j)
-      for (int i = 0; i < 9; ++i) B.Zl[(size_t)j * kZlPitch + i] = (R)0;
+      for (int i = 0; i < 9; ++i) zl_at(B, j, i) = (R)0;
     return;
   }
   // V, v and the Y / Z products accumulate in the storage precision R; the 3x3
@@ -300,13 +309,12 @@ __device__ __forceinline__ void point_system(const Prob& P, const StateView& st,
         Y[3 * a + 2] += (ga * j2 + gb * j5) * w;
       }
     }
-    R* Zl = B.Zl + (size_t)j * kZlPitch;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const R y0 = Y[3 * a], y1 = Y[3 * a + 1], y2 = Y[3 * a + 2];
-      Zl[3 * a + 0] = ok ? y0 * l00 + y1 * l10 + y2 * l20 : (R)0;
-      Zl[3 * a + 1] = ok ? y1 * l11 + y2 * l21 : (R)0;
-      Zl[3 * a + 2] = ok ? y2 * l22 : (R)0;
+      zl_at(B, j, 3 * a + 0) = ok ? y0 * l00 + y1 * l10 + y2 * l20 : (R)0;
+      zl_at(B, j, 3 * a + 1) = ok ? y1 * l11 + y2 * l21 : (R)0;
+      zl_at(B, j, 3 * a + 2) = ok ? y2 * l22 : (R)0;
     }
   }
 }
@@ -576,7 +584,7 @@ static __device__ __noinline__ void point_system_mixed_ill(const Prob& P, const 
       for (int i = 0; i < 9; ++i) B.gsub[(size_t)k * 9 + i] = 0.0f;
     }
     for (uint32_t j = S.lens_ptr[p]; j < S.lens_ptr[p + 1]; ++j)
-      for (int i = 0; i < 9; ++i) B.Zl[(size_t)j * kZlPitch + i] = 0.0f;
+      for (int i = 0; i < 9; ++i) zl_at(B, j, i) = 0.0f;
     return;
   }
   const double zv0 = L[0] * v[0] + L[1] * v[1] + L[3] * v[2];
@@ -642,13 +650,12 @@ static __device__ __noinline__ void point_system_mixed_ill(const Prob& P, const 
         Y[3 * a + 2] += (ga * j2 + gb * j5) * w;
       }
     }
-    float* Zl = B.Zl + (size_t)j * kZlPitch;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const double y0 = Y[3 * a], y1 = Y[3 * a + 1], y2 = Y[3 * a + 2];
-      Zl[3 * a + 0] = (float)(y0 * L[0] + y1 * L[1] + y2 * L[3]);
-      Zl[3 * a + 1] = (float)(y1 * L[2] + y2 * L[4]);
-      Zl[3 * a + 2] = (float)(y2 * L[5]);
+      zl_at(B, j, 3 * a + 0) = (float)(y0 * L[0] + y1 * L[1] + y2 * L[3]);
+      zl_at(B, j, 3 * a + 1) = (float)(y1 * L[2] + y2 * L[4]);
+      zl_at(B, j, 3 * a + 2) = (float)(y2 * L[5]);
     }
   }
 }
@@ -782,7 +789,7 @@ __device__ __forceinline__ void point_mixed_finish(
   if (!sum) {  // fewer than two observations (ba.rs:238)
     B.kept[p] = 0;
     for (uint32_t j = l0; j < l1; ++j)
-      for (int i = 0; i < 9; ++i) B.Zl[(size_t)j * kZlPitch + i] = 0.0f;
+      for (int i = 0; i < 9; ++i) zl_at(B, j, i) = 0.0f;
     return;
   }
   double V[6], v[3];
@@ -865,13 +872,12 @@ __device__ __forceinline__ void point_mixed_finish(
         Y[3 * a + 2] += (ga * j2 + gb * j5) * w;
       }
     }
-    float* Zl = B.Zl + (size_t)j * kZlPitch;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const float y0 = Y[3 * a], y1 = Y[3 * a + 1], y2 = Y[3 * a + 2];
-      Zl[3 * a + 0] = y0 * l00 + y1 * l10 + y2 * l20;
-      Zl[3 * a + 1] = y1 * l11 + y2 * l21;
-      Zl[3 * a + 2] = y2 * l22;
+      zl_at(B, j, 3 * a + 0) = y0 * l00 + y1 * l10 + y2 * l20;
+      zl_at(B, j, 3 * a + 1) = y1 * l11 + y2 * l21;
+      zl_at(B, j, 3 * a + 2) = y2 * l22;
     }
   }
 }
@@ -1837,21 +1843,21 @@ __device__ __forceinline__ void load_Z(const IterBufs<R>& B, uint32_t k, R* z) {
     load_Z18(B.Z + (size_t)k * B.zpitch, z);
 }
 // A lens entry's nine values.
-__device__ __forceinline__ void load_Zl(const double* s, double* z) {
-  const double2* v = reinterpret_cast<const double2*>(s);
+__device__ __forceinline__ void load_Zl(const IterBufs<double>& B, size_t j, double* z) {
+  const double2* v = reinterpret_cast<const double2*>(B.Zl + j * kZlPitch);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const double2 t = __ldg(v + i);
     z[2 * i] = t.x, z[2 * i + 1] = t.y;
   }
-  z[8] = __ldg(s + 8);
+  z[8] = __ldg(B.Zl9 + j);
 }
-__device__ __forceinline__ void load_Zl(const float* s, float* z) {
-  const float4* v = reinterpret_cast<const float4*>(s);
+__device__ __forceinline__ void load_Zl(const IterBufs<float>& B, size_t j, float* z) {
+  const float4* v = reinterpret_cast<const float4*>(B.Zl + j * kZlPitch);
   const float4 a = __ldg(v), b = __ldg(v + 1);
   z[0] = a.x, z[1] = a.y, z[2] = a.z, z[3] = a.w;
   z[4] = b.x, z[5] = b.y, z[6] = b.z, z[7] = b.w;
-  z[8] = __ldg(s + 8);
+  z[8] = __ldg(B.Zl9 + j);
 }
 
 // What the pairs of a destination block are, and so which of its 36 entries
@@ -1916,14 +1922,14 @@ __device__ __forceinline__ void schur_segment(const Prob& P, const StructView& S
     if constexpr (O::kRows == 6)
       load_Z(B, ea, za);
     else
-      load_Zl(B.Zl + (size_t)(ea - P.no) * kZlPitch, za);
+      load_Zl(B, (size_t)(ea - P.no), za);
     if constexpr (O::kSym) {
 #pragma unroll
       for (int t = 0; t < 3 * O::kRows; ++t) zb[t] = za[t];
     } else if constexpr (O::kCols == 6) {
       load_Z(B, eb, zb);
     } else {
-      load_Zl(B.Zl + (size_t)(eb - P.no) * kZlPitch, zb);
+      load_Zl(B, (size_t)(eb - P.no), zb);
     }
     int n = 0;
 #pragma unroll
@@ -2345,7 +2351,9 @@ __global__ void backsub_kernel(Prob P, StructView S, StateView cur, StateView tr
       }
     }
     for (uint32_t j = S.lens_ptr[p]; j < S.lens_ptr[p + 1]; ++j) {
-      const R* Z = B.Zl + (size_t)j * kZlPitch;
+      R Z[9];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) Z[i] = zl_at(B, j, i);
       const R* d = B.x + 6 * (size_t)P.grp_blk[S.lens_grp[j]];
 #pragma unroll
       for (int r = 0; r < 3; ++r) {

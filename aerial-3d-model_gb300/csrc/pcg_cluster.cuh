@@ -27,6 +27,17 @@
 // does (the same sums in the same order, so the same α), then its rows of
 // E^-1 w, so the step adds no CTA barrier to the iteration.
 //
+// S blocks beyond the shared memory are read every iteration: of 1200
+// cameras 58 %, 220 KB a CTA, for which the loads of 16 bytes a lane at 144
+// bytes' distance (a cache line a lane, and a small L1 beside 227 KB of shared
+// memory) took half of the iteration.  They are turned once per solve into
+// runs that a warp loads in whole lines: 29.2 -> 22.3 us per iteration (two
+// levels, 16 CTAs).  A batch with more models than clusters of one CTA an SM
+// runs two CTAs an SM on half the shared memory, the large models first: an
+// iteration waits for its barriers most of the time, and a second cluster
+// fills the wait.  32 models of 20 to 400 cameras, 12 CTAs each: 31.5 -> 20.7 ms
+// of a solve's PCG.
+//
 // Every CTA of a cluster executes the same sequence of cluster barriers:
 // loop exits depend only on reduced scalars, which every CTA computes from
 // the same partials in the same order (bit-identical), and the kernel has no
@@ -79,6 +90,7 @@ struct CgArgs {
   const uint32_t* diag_pos; // [nb]
   uint32_t cap_rows;        // row-state capacity (same in every CTA)
   uint32_t cap_blocks;      // cached S blocks per CTA (the rest read from global)
+  uint32_t cap_slots;       // blocks per CTA whose cache slot is in shared memory
   const int32_t* active;
   int32_t* iters;
   int32_t max_iter;
@@ -103,6 +115,8 @@ struct CgArgs {
   const uint32_t* sub_ent;
   uint32_t cap_cache;        // cache slots per CTA
   const int32_t* cap = nullptr;  // [nm] or null: per-model iteration cap (below max_iter)
+  float* turned = nullptr;   // [nz * 36]: where the blocks that are not cached are turned
+  const int32_t* order = nullptr;  // [grid / cluster]: the cluster's model, largest first
   unsigned* err = nullptr;   // device error bits (a staging wait that gave up)
   long long spin = 0;        // limit of that wait, in SM clock cycles
 };
@@ -146,9 +160,19 @@ __device__ __forceinline__ bool cg_bulk_wait(uint64_t* bar, long long spin) {
   }
 }
 
-inline size_t cg_smem_bytes(uint32_t cap_rows, uint32_t cap_blocks, uint32_t cap_cache) {
-  return (size_t)cap_rows * kCgRow * 4 + (size_t)cap_blocks * (36 * 4 + 4) +
-         (size_t)cap_cache * kCgCache * 4;
+// A block's cache slot as kept in shared memory: the CTA's own row in the low
+// 15 bits under bit 15, else the slot (a slot takes 96 bytes and a row 320 of
+// the same shared memory, so both numbers stay far below 2^15).
+constexpr uint32_t kCgOwnSlot = 0x8000u;
+__device__ __forceinline__ uint32_t cg_slot16(uint32_t e) {
+  return ((e & kCgOwnRow) ? kCgOwnSlot : 0u) | (e & 0x7fffu);
+}
+// Slots in shared memory, in whole 16-byte words.
+inline size_t cg_slot_bytes(uint32_t cap_slots) { return ((size_t)cap_slots * 2 + 15) / 16 * 16; }
+inline size_t cg_smem_bytes(uint32_t cap_rows, uint32_t cap_blocks, uint32_t cap_cache,
+                            uint32_t cap_slots) {
+  return (size_t)cap_rows * kCgRow * 4 + (size_t)cap_blocks * (36 * 4) +
+         (size_t)cap_cache * kCgCache * 4 + cg_slot_bytes(cap_slots);
 }
 
 // Extra shared memory of the two-level form, in floats: per row W (42); per
@@ -390,8 +414,22 @@ __device__ __forceinline__ void cg_push_row(cgx::cluster_group& cl, float* cache
   }
 }
 
-template <bool kCoarse, int kThreads>
-static __global__ void __launch_bounds__(kThreads) pcg_cluster_kernel(CgArgs A) {
+// A block's 36 values from a turned run of up to 32 blocks that starts at
+// block c0 of a row that ends at block b1: this CTA's warps wrote them before
+// the cluster barrier after the staging.
+__device__ __forceinline__ void cg_load_turned(const float* turned, uint32_t c0, uint32_t b1,
+                                               int i, float (&m)[36]) {
+  const uint32_t n = b1 - c0 < 32u ? b1 - c0 : 32u;
+  const float4* v = reinterpret_cast<const float4*>(turned) + (size_t)c0 * 9 + i;
+#pragma unroll
+  for (int t = 0; t < 9; ++t) {
+    const float4 w = v[t * n];
+    m[4 * t] = w.x, m[4 * t + 1] = w.y, m[4 * t + 2] = w.z, m[4 * t + 3] = w.w;
+  }
+}
+
+template <bool kCoarse, int kThreads, int kCtas>
+static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgArgs A) {
   constexpr int kCgWarps = kThreads / 32;
   __shared__ float wsm[kCgWarps * 4];
   __shared__ DFloat inbox[3][kCgMaxCluster][4];  // reduction inboxes (push)
@@ -401,28 +439,32 @@ static __global__ void __launch_bounds__(kThreads) pcg_cluster_kernel(CgArgs A) 
   __shared__ uint64_t stage_bar;  // completion of the S blocks' bulk copy
   extern __shared__ __align__(16) unsigned char cg_smem[];
   cgx::cluster_group cl = cgx::this_cluster();
-  const CgJob J = A.jobs[blockIdx.x];
+  // clusters are 1-D: the cluster's CTAs are consecutive blocks
+  const uint32_t csz = (uint32_t)cl.num_blocks();
+  const uint32_t job = (uint32_t)A.order[blockIdx.x / csz] * csz + blockIdx.x % csz;
+  const CgJob J = A.jobs[job];
   if (!A.active[J.model]) return;  // uniform over the cluster
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t nrows = J.row1 - J.row0;
   const uint32_t B0 = A.row_ptr[J.row0];
   const uint32_t nblk = A.row_ptr[J.row1] - B0;
   const uint32_t ncached = nblk < A.cap_blocks ? nblk : A.cap_blocks;
-  // Shared memory: row state | cached S blocks | neighbour cache | cached
+  const uint32_t nslots = nblk < A.cap_slots ? nblk : A.cap_slots;
+  // Shared memory: row state | cached S blocks | neighbour cache | the
   // blocks' cache slots | two-level form: W per row, E^-1 rows and c per own
   // group, the model's group sums of W^T r (two buffers) and W^T q.
   float* rs = reinterpret_cast<float*>(cg_smem);
   float* sS = rs + (size_t)A.cap_rows * kCgRow;
   float* cache = sS + (size_t)A.cap_blocks * 36;
-  uint32_t* sL = reinterpret_cast<uint32_t*>(cache + (size_t)A.cap_cache * kCgCache);
-  float* sW = reinterpret_cast<float*>(sL + A.cap_blocks);
+  uint16_t* sL = reinterpret_cast<uint16_t*>(cache + (size_t)A.cap_cache * kCgCache);
+  float* sW = reinterpret_cast<float*>(sL + ((size_t)A.cap_slots + 7) / 8 * 8);
   float* sEi = sW + (size_t)A.cap_rows * 42;
   const size_t gsz = (size_t)A.cap_groups * kCoarseModes;
   float* scf = sEi + gsz * A.cap_dim;        // c, own outputs
   float* wall_r = scf + gsz;                  // [2][D]
   float* wall_q = wall_r + 2 * (size_t)A.cap_dim;  // [D]
-  const int32_t cg0 = kCoarse ? A.job_g0[blockIdx.x] : 0;
-  const int32_t ngr = kCoarse ? A.job_g1[blockIdx.x] - cg0 : 0;
+  const int32_t cg0 = kCoarse ? A.job_g0[job] : 0;
+  const int32_t ngr = kCoarse ? A.job_g1[job] - cg0 : 0;
   const int32_t goff = kCoarse ? kCoarseModes * (cg0 - A.model_g0[J.model]) : 0;
   const int32_t lens = A.lens_row[J.model];
   // the model's coarse dimension and this CTA's coarse outputs (two-level form)
@@ -431,7 +473,8 @@ static __global__ void __launch_bounds__(kThreads) pcg_cluster_kernel(CgArgs A) 
   {
     if (threadIdx.x == 0 && ncached > 0)
       cg_bulk_stage(&stage_bar, sS, A.S + (size_t)B0 * 36, ncached * 36u * 4u);
-    for (uint32_t t = threadIdx.x; t < ncached; t += blockDim.x) sL[t] = A.blk_slot[B0 + t];
+    for (uint32_t t = threadIdx.x; t < nslots; t += blockDim.x)
+      sL[t] = (uint16_t)cg_slot16(A.blk_slot[B0 + t]);
     // p(prev) of iteration 0 is 0 in every cached row; the z values arrive
     // by push after the first cluster barrier.
     for (uint32_t t = threadIdx.x; t < A.cap_cache * kCgCache; t += blockDim.x) cache[t] = 0.0f;
@@ -466,6 +509,29 @@ static __global__ void __launch_bounds__(kThreads) pcg_cluster_kernel(CgArgs A) 
         const int o = t / D, col = t % D;
         sEi[(size_t)o * A.cap_dim + col] =
             Ei[(size_t)(kCoarseModes * (cg0 - gm0) + o) * D + col];
+      }
+    }
+  }
+  // The blocks that shared memory has no room for, turned once per solve: the
+  // 32 blocks that a warp multiplies at a time lie block by block, and lanes
+  // that each load one block's pieces touch 32 cache lines a load; turned,
+  // piece t of the blocks side by side, a load is 512 bytes in a row.
+  if (ncached < nblk) {
+    __syncthreads();
+    for (uint32_t lr = warp; lr < nrows; lr += kCgWarps) {
+      const float* st = rs + (size_t)lr * kCgRow;
+      const uint32_t b0 = (uint32_t)__float_as_int(st[kCgIdx]);
+      const uint32_t b1 = (uint32_t)__float_as_int(st[kCgIdx + 1]);
+      for (uint32_t c0 = b0; c0 < b1; c0 += 32) {
+        const uint32_t n = b1 - c0 < 32u ? b1 - c0 : 32u;
+        if (c0 + n - B0 <= ncached) continue;
+        const float4* src = reinterpret_cast<const float4*>(A.S) + (size_t)c0 * 9;
+        float4* dst = reinterpret_cast<float4*>(A.turned) + (size_t)c0 * 9;
+#pragma unroll
+        for (int u = 0; u < 9; ++u) {
+          const uint32_t e = 32 * u + lane;
+          if (e < 9 * n) dst[(e % 9) * n + e / 9] = __ldg(src + e);
+        }
       }
     }
   }
@@ -562,10 +628,10 @@ static __global__ void __launch_bounds__(kThreads) pcg_cluster_kernel(CgArgs A) 
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       for (uint32_t k = b0 + lane; k < b1; k += 32) {
         const uint32_t kk = k - B0;
-        const uint32_t slot = kk < ncached ? sL[kk] : __ldg(A.blk_slot + k);
+        const uint32_t slot = kk < nslots ? sL[kk] : cg_slot16(__ldg(A.blk_slot + k));
         float pp[6];
-        if (slot & kCgOwnRow) {  // one of this CTA's rows: its row state
-          const float* o = CGROW(slot & ~kCgOwnRow);
+        if (slot & kCgOwnSlot) {  // one of this CTA's rows: its row state
+          const float* o = CGROW(slot & ~kCgOwnSlot);
 #pragma unroll
           for (int j = 0; j < 6; ++j) pp[j] = o[kCgZ + j] + o[kCgP + 6 * prv + j] * bf;
         } else {
@@ -578,7 +644,10 @@ static __global__ void __launch_bounds__(kThreads) pcg_cluster_kernel(CgArgs A) 
           pp[3] = z0.w + q0.w * bf, pp[4] = z1.x + q1.x * bf, pp[5] = z1.y + q1.y * bf;
         }
         float m[36];
-        load_block(kk < ncached ? sS + (size_t)kk * 36 : A.S + (size_t)k * 36, m);
+        if (kk < ncached)
+          load_block(sS + (size_t)kk * 36, m);
+        else
+          cg_load_turned(A.turned, k - lane, b1, lane, m);
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
           float s = acc[i];

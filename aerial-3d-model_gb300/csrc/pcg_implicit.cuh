@@ -41,6 +41,7 @@ struct ImpArgs {
   StructView SV;
   const R* Z;        // [no][18], or null: recomputed (mixed form, from zsrc)
   const R* Zl;       // [nl][kZlPitch]
+  const R* Zl9;      // [nl]
   const uint8_t* kept;
   const R* own;      // [nb][36]: A_c (cameras) / A_g (lens row)
   const double* camX;  // [nc][18]: X_c = sum w Jc^T Jg (6x3)
@@ -162,7 +163,9 @@ __global__ void __launch_bounds__(kPcgThreads) pcg_implicit_kernel(ImpArgs<R> A)
           }
         }
         for (uint32_t j = A.SV.lens_ptr[pt]; j < A.SV.lens_ptr[pt + 1]; ++j) {
-          const R* Zj = A.Zl + kZlPitch * (size_t)j;
+          R Zj[9];
+#pragma unroll
+          for (int i = 0; i < 9; ++i) Zj[i] = zl_at(A, j, i);
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
             t0 += Zj[3 * i] * pg[i];
@@ -171,7 +174,9 @@ __global__ void __launch_bounds__(kPcgThreads) pcg_implicit_kernel(ImpArgs<R> A)
           }
         }
         for (uint32_t j = A.SV.lens_ptr[pt]; j < A.SV.lens_ptr[pt + 1]; ++j) {
-          const R* Zj = A.Zl + kZlPitch * (size_t)j;
+          R Zj[9];
+#pragma unroll
+          for (int i = 0; i < 9; ++i) Zj[i] = zl_at(A, j, i);
 #pragma unroll
           for (int i = 0; i < 3; ++i)
             wl[i] += (double)(Zj[3 * i] * t0 + Zj[3 * i + 1] * t1 + Zj[3 * i + 2] * t2);
@@ -317,7 +322,9 @@ __global__ void lens_diag_kernel(StructView S, IterBufs<R> B, double* lens_part)
 #pragma unroll
   for (int i = 0; i < 9; ++i) s[i] = 0.0;
   for (int64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-    const R* Zj = B.Zl + kZlPitch * (size_t)j;
+    R Zj[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) Zj[i] = zl_at(B, j, i);
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll

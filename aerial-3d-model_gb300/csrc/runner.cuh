@@ -128,6 +128,8 @@ struct ClusterPlan {
   std::vector<CgJob> jobs;
   std::vector<uint32_t> row_loc;
   uint32_t max_rows = 0, max_blocks = 0;
+  uint32_t need_blocks = 0;    // most blocks a CTA multiplies (of the lens row only the diagonal)
+  std::vector<int32_t> order;  // the models, most blocks first
 };
 
 inline bool plan_cluster(const Context& ctx, const std::vector<uint32_t>& row_ptr,
@@ -135,7 +137,7 @@ inline bool plan_cluster(const Context& ctx, const std::vector<uint32_t>& row_pt
                          ClusterPlan& pl) {
   pl.jobs.clear();
   pl.row_loc.assign(row_ptr.size() - 1, 0);
-  pl.max_rows = pl.max_blocks = 0;
+  pl.max_rows = pl.max_blocks = pl.need_blocks = 0;
   for (int64_t m = 0; m < ctx.nm; ++m) {
     const uint32_t r0 = ctx.h_blk0[m], r1 = ctx.h_blk0[m + 1];
     std::vector<int64_t> rc(r1 - r0);
@@ -159,9 +161,18 @@ inline bool plan_cluster(const Context& ctx, const std::vector<uint32_t>& row_pt
       pl.jobs.push_back(CgJob{(int32_t)m, start, row});
       pl.max_rows = std::max(pl.max_rows, row - start);
       pl.max_blocks = std::max(pl.max_blocks, row_ptr[row] - row_ptr[start]);
+      const bool ends = row > start && lens_row[m] == (int32_t)row - 1;  // with the lens row
+      pl.need_blocks = std::max(pl.need_blocks, row_ptr[row - (ends ? 1 : 0)] - row_ptr[start]);
     }
     if (row != r1) return false;
   }
+  // A cluster that starts when others end should be a small one: the models
+  // in descending order of their blocks.
+  pl.order.resize((size_t)ctx.nm);
+  for (int64_t m = 0; m < ctx.nm; ++m) pl.order[(size_t)m] = (int32_t)m;
+  auto blocks = [&](int32_t m) { return row_ptr[ctx.h_blk0[m + 1]] - row_ptr[ctx.h_blk0[m]]; };
+  std::stable_sort(pl.order.begin(), pl.order.end(),
+                   [&](int32_t a, int32_t b) { return blocks(a) > blocks(b); });
   return true;
 }
 
@@ -307,13 +318,18 @@ void h2d(DevBuf<T>& d, const std::vector<T>& h, cudaStream_t s) {
 
 inline int64_t at_least_1(int64_t n) { return n > 0 ? n : 1; }
 
-// The cluster PCG kernel for the coarse flag and the threads per CTA.
+// The cluster PCG kernel for the coarse flag, the threads per CTA and (512
+// threads) the CTAs per SM.
 using CgKernel = void (*)(CgArgs);
-inline CgKernel cg_kernel(bool coarse, int threads) {
+inline CgKernel cg_kernel(bool coarse, int threads, bool two) {
   if (threads == kCgThreadsWide)
-    return coarse ? pcg_cluster_kernel<true, kCgThreadsWide>
-                  : pcg_cluster_kernel<false, kCgThreadsWide>;
-  return coarse ? pcg_cluster_kernel<true, kCgThreads> : pcg_cluster_kernel<false, kCgThreads>;
+    return coarse ? pcg_cluster_kernel<true, kCgThreadsWide, 1>
+                  : pcg_cluster_kernel<false, kCgThreadsWide, 1>;
+  if (two)
+    return coarse ? pcg_cluster_kernel<true, kCgThreads, 2>
+                  : pcg_cluster_kernel<false, kCgThreads, 2>;
+  return coarse ? pcg_cluster_kernel<true, kCgThreads, 1>
+                : pcg_cluster_kernel<false, kCgThreads, 1>;
 }
 
 }  // namespace detail
@@ -505,9 +521,11 @@ struct LmEngine {
   int32_t imp_ncta = 0;
   // Cluster-resident PCG (mixed form).
   bool use_cluster = false;
+  bool cl_two = false;  // two of the cluster kernel's CTAs per SM
   int cl_size = 0;
   int cl_threads = kCgThreads;  // threads per CTA of the cluster kernel
   DevBuf<CgJob> cg_jobs;
+  DevBuf<int32_t> cg_order;
   DevBuf<uint32_t> cg_loc, cg_slot, cg_subp, cg_sube;
   std::vector<uint32_t> h_col_idx, h_diag_pos;  // host copies for the cache plan
   CgArgs ca{};
@@ -657,7 +675,7 @@ struct LmEngine {
       Z.release();
     else
       Z.alloc(at_least_1(no) * (z24 ? 24 : 18) + 4, s);
-    Zl.alloc(at_least_1(SB.nl) * kZlPitch, s);
+    Zl.alloc(at_least_1(SB.nl) * 9, s);
     ptL.alloc(at_least_1(np) * 6, s), ptzv.alloc(at_least_1(np) * 3, s);
     kept.alloc(at_least_1(np), s);
     camU.alloc(at_least_1(nc) * 21, s), camgj.alloc(at_least_1(nc) * 6, s);
@@ -683,7 +701,8 @@ struct LmEngine {
     // Two-level PCG (mixed form): the FP64 values of S for the coarse matrix,
     // written by every assembly (the autotuner assembles before it plans).
     if (sizeof(R) == 4 && o.coarse && !implicit) c_S64.alloc(at_least_1(SB.nz) * 36, s);
-    B = IterBufs<R>{lin, gsub, Z, Zl, ptL, ptzv, kept, camU, camgj, camgs, camX, caml,
+    B = IterBufs<R>{lin, gsub, Z, Zl, Zl + at_least_1(SB.nl) * kZlPitch, ptL, ptzv, kept, camU,
+                    camgj, camgs, camX, caml,
                     grpU, grpg, part, S, pre, g, x, cost_part, ptf.p};
     B.zpos = sizeof(R) == 4 && SB.z_by_camera ? SB.cam_pos.p : nullptr;
     B.zpitch = B.zpos ? 24 : 18;
@@ -907,7 +926,7 @@ struct LmEngine {
     bar_base.zero();
     pcg_part.alloc(kParts * (size_t)imp_ncta, s);
     z.alloc(detail::at_least_1(ctx.nb) * 6, s), p.alloc(detail::at_least_1(ctx.nb) * 12, s);
-    ia = ImpArgs<R>{bar, bar_base, pcg_part, imp_ncta, ctx.err, P, SV, B.Z, Zl, kept, own, camX,
+    ia = ImpArgs<R>{bar, bar_base, pcg_part, imp_ncta, ctx.err, P, SV, B.Z, B.Zl, B.Zl9, kept, own, camX,
                     pre, g, x, rbuf, z, p, qbuf, tbuf, h_lens[0], (int32_t)ctx.nb, pcg_iters,
                     pcg_limit, o.pcg_tol, o.wait_limit};
     ia.cap = pcg_cap;
@@ -967,7 +986,7 @@ struct LmEngine {
           "attr");
     const bool coarse = o.coarse != 0;
     if (threads != kCgThreadsWide) threads = kCgThreads;
-    const detail::CgKernel kfn = detail::cg_kernel(coarse, threads);
+    const detail::CgKernel kfn = detail::cg_kernel(coarse, threads, false);
     cudaFuncAttributes fa{};
     check(cudaFuncGetAttributes(&fa, kfn), "func attr");
     const size_t avail = (size_t)smem_optin - fa.sharedSizeBytes;
@@ -982,6 +1001,7 @@ struct LmEngine {
     if (!detail::plan_cluster(ctx, SB.h_row_ptr, h_lens, csize, rows_cap, cp))
       return unusable("a model has too many block rows for one cluster");
     if (cp.max_blocks == 0 && cp.max_rows == 0) return unusable("empty plan");
+    if (2 * SB.nsub < SB.nz) return unusable("blocks without sub-segments");
     detail::CoarsePlan gp;
     size_t coarse_bytes = 0;
     if (coarse) {
@@ -1015,10 +1035,12 @@ struct LmEngine {
     const size_t cache_bytes = (size_t)kp.cap * kCgCache * 4;
     if (row_bytes + coarse_bytes + cache_bytes >= avail)
       return unusable("row state and neighbour cache do not fit");
-    const uint32_t cap_blocks = (uint32_t)std::min<size_t>(
-        cp.max_blocks, (avail - row_bytes - coarse_bytes - cache_bytes) / (36 * 4 + 4));
-    const size_t smem = cg_smem_bytes(cp.max_rows, cap_blocks, kp.cap) + coarse_bytes;
-    check(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    const size_t fixed_bytes = row_bytes + coarse_bytes + cache_bytes;
+    // Whether the clusters serve: with every S block cached that fits beside a
+    // slot of 4 bytes each.
+    size_t smem = fixed_bytes +
+                  std::min<size_t>(cp.max_blocks, (avail - fixed_bytes) / (36 * 4 + 4)) * (36 * 4 + 4);
+    check(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)avail),
           "cluster smem");
     if (csize > 8)
       check(cudaFuncSetAttribute(kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
@@ -1047,6 +1069,41 @@ struct LmEngine {
     // resident at once (one wave); otherwise models would queue behind each
     // other while the grid kernel runs them all together.
     if (!required && !prefer_cluster && (int64_t)nclusters < ctx.nm) return false;
+    // What a CTA keeps within `bytes` of shared memory: the cache slots of its
+    // blocks (2 bytes each), then S blocks.
+    uint32_t cap_slots = 0, cap_blocks = 0;
+    auto fill = [&](size_t bytes) {
+      cap_slots = (uint32_t)std::min<size_t>(cp.need_blocks, (bytes - fixed_bytes) / 16 * 8);
+      cap_blocks = (uint32_t)std::min<size_t>(
+          cp.need_blocks, (bytes - fixed_bytes - cg_slot_bytes(cap_slots)) / (36 * 4));
+      return cg_smem_bytes(cp.max_rows, cap_blocks, kp.cap, cap_slots) + coarse_bytes;
+    };
+    smem = fill(avail);
+    // More models than clusters at a time: two CTAs an SM, each with the S
+    // blocks that half the shared memory holds (the rest turned in global
+    // memory), when that lets more clusters run.
+    bool two = false;
+    if ((int64_t)nclusters < ctx.nm && threads == kCgThreads) {
+      int per_sm = 0, reserved = 0, nhalf = 0;
+      check(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx.device),
+            "attr");
+      check(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, ctx.device),
+            "attr");
+      const detail::CgKernel kf2 = detail::cg_kernel(coarse, threads, true);
+      const size_t half = ((size_t)per_sm / 2 - (size_t)reserved - fa.sharedSizeBytes) / 16 * 16;
+      if (half < smem && fixed_bytes + cg_slot_bytes(cp.need_blocks) <= half) {
+        check(cudaFuncSetAttribute(kf2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)half),
+              "cluster smem");
+        if (csize > 8)
+          check(cudaFuncSetAttribute(kf2, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+                "cluster size");
+        cfg.dynamicSmemBytes = half;
+        if (cudaOccupancyMaxActiveClusters(&nhalf, kf2, &cfg) != cudaSuccess) cudaGetLastError();
+        two = nhalf > nclusters;
+        if (two) smem = fill(half);
+      }
+    }
+    detail::h2d(cg_order, cp.order, s);
     detail::h2d(cg_jobs, cp.jobs, s);
     detail::h2d(cg_loc, cp.row_loc, s);
     detail::h2d(cg_slot, kp.blk_slot, s);
@@ -1054,7 +1111,8 @@ struct LmEngine {
     detail::h2d(cg_sube, kp.sub_ent, s);
     ca = CgArgs{cg_jobs, cg_loc, SB.row_ptr, SB.col_idx, (const float*)S.p, (const float*)pre.p,
                 (const float*)g.p, (float*)x.p, lens_row, lens_pos, SB.diag_pos, cp.max_rows,
-                cap_blocks, active, pcg_iters, pcg_limit, o.pcg_tol};
+                cap_blocks, cap_slots, active, pcg_iters, pcg_limit, o.pcg_tol};
+    ca.order = cg_order;
     ca.cap = pcg_cap;
     ca.blk_slot = cg_slot, ca.sub_ptr = cg_subp, ca.sub_ent = cg_sube, ca.cap_cache = kp.cap;
     ca.err = ctx.err, ca.spin = o.wait_limit;
@@ -1084,6 +1142,7 @@ struct LmEngine {
     }
     check(cudaStreamSynchronize(s), "sync");
     cg_smem = smem;
+    cl_two = two;
     cl_size = csize;
     cl_threads = threads;
     use_cluster = true;
@@ -1378,7 +1437,11 @@ struct LmEngine {
       cfg.stream = s;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
-      check(cudaLaunchKernelEx(&cfg, detail::cg_kernel(use_coarse, cl_threads), ca),
+      // The blocks that are not cached are turned into the sub-segments' sums
+      // (at least 36 FP64 values for a pair of mirrored blocks), which the
+      // assembly has read and the next Schur pass writes anew.
+      ca.turned = (float*)part.p;
+      check(cudaLaunchKernelEx(&cfg, detail::cg_kernel(use_coarse, cl_threads, cl_two), ca),
             "pcg cluster launch");
     } else {
       void* args[] = {&pa};
