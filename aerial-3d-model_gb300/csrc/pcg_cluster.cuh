@@ -7,15 +7,15 @@
 // blocks); each CTA keeps its rows' state (x, r, z, two buffers of p, q and
 // the block-Jacobi inverse) and its rows' S blocks in shared memory for the
 // whole solve.  Every value another CTA needs is pushed to it: a CTA keeps a
-// cache of the neighbour rows its blocks multiply (z_j and both buffers of
-// p_j), and each row's owner stores the row's new z and p into the caches of
-// the CTAs that read it (a host-built subscriber list) before the cluster
-// barrier after which they are read.  Remote loads would be round trips a
+// cache of the neighbour rows its blocks multiply (z_j and p_j), and each
+// row's owner stores the row's new z into the caches of the CTAs that read it
+// (a host-built subscriber list) before the cluster barrier after which they
+// are read; every CTA then forms p_j = z_j + β p_j of its cached rows itself,
+// once an iteration.  Remote loads would be round trips a
 // warp waits on (~4.5k cycles when its lanes read from 16 CTAs); remote
 // stores complete behind the barrier's release.  The two reductions of an
 // iteration meet at hardware cluster barriers: no global memory traffic and
-// no software spin inside the iteration.  The iteration is the reference's,
-// with p_j = z_j + β p_j(prev) formed on the fly as in the grid kernel.
+// no software spin inside the iteration.
 //
 // Two-level form (coarse correction z = B^-1 r + W E^-1 W^T r): the coarse
 // vector of the next residual, w = W^T r_{k+1}, is formed as W^T r_k −
@@ -23,20 +23,26 @@
 // barrier (α is known right after it), so an iteration still needs only two
 // cluster reductions: p·q (then α, the coarse gather and c = E^-1 w), and
 // r·r with r·z (then β).  The coarse step runs on the warps beside warp 0
-// after the p·q barrier: each of them sums the inbox and forms α as warp 0
-// does (the same sums in the same order, so the same α), then its rows of
-// E^-1 w, so the step adds no CTA barrier to the iteration.
+// after the p·q barrier, when every warp has formed α.
 //
 // S blocks beyond the shared memory are read every iteration: of 1200
 // cameras 58 %, 220 KB a CTA, for which the loads of 16 bytes a lane at 144
 // bytes' distance (a cache line a lane, and a small L1 beside 227 KB of shared
 // memory) took half of the iteration.  They are turned once per solve into
-// runs that a warp loads in whole lines: 29.2 -> 22.3 us per iteration (two
-// levels, 16 CTAs).  A batch with more models than clusters of one CTA an SM
+// runs that a warp loads in whole lines: 29.2 -> 22.3 us per iteration (1200
+// cameras, two levels, 16 CTAs).  A batch with more models than clusters of one CTA an SM
 // runs two CTAs an SM on half the shared memory, the large models first: an
 // iteration waits for its barriers most of the time, and a second cluster
 // fills the wait.  32 models of 20 to 400 cameras, 12 CTAs each: 31.5 -> 20.7 ms
 // of a solve's PCG.
+//
+// What is left is latency: three or four rows a warp, one after the other, and
+// two exchanges.  A row of S p is a warp's work, a lane a block; what is six
+// values a row (p.q, the update of x, r and z, their pushes) is done for five
+// rows at a time, and p is formed per cached row instead of pushed and formed
+// per block.  Two rows of S p at once in a warp's registers were slower (the
+// longer code: 7.1 -> 7.6 ms).  Together 22.3 -> 15.8 us per iteration (1200
+// cameras), 11.0 -> 9.0 us (500), 20.7 -> 18.8 ms (the batch).
 //
 // Every CTA of a cluster executes the same sequence of cluster barriers:
 // loop exits depend only on reduced scalars, which every CTA computes from
@@ -61,15 +67,23 @@ constexpr int kCgThreads = 512;
 constexpr int kCgThreadsWide = 1024;
 constexpr int kCgMaxCluster = 16;
 // Row state in floats: x r z p0 p1 q (6 each) | M (36) | the row's first and
-// end block, its lens block, its coarse group slot and its subscriber range
-// (int bits) | pad.  Accessed one component per lane.
+// end block, its lens block, its coarse group slot and number of subscribers,
+// its first subscriber (int bits).  Accessed one component per lane, or one
+// row per lane (the pitch is odd: 32 rows in 32 banks).
 constexpr int kCgX = 0, kCgR = 6, kCgZ = 12, kCgP = 18, kCgQ = 30, kCgM = 36, kCgIdx = 72;
+constexpr int kCgPitch = 77;
+// Floats of shared memory per row.
 constexpr int kCgRow = 80;
 // A block's column is one of the CTA's own rows when its slot carries this
 // bit (the low bits are the local row), else a slot of the neighbour cache.
 constexpr uint32_t kCgOwnRow = 0x80000000u;
-// Neighbour cache slot in floats: z (8, 6 used) | p buffer 0 (8) | p buffer 1.
-constexpr int kCgCache = 24;
+// Neighbour cache in floats per slot: z, and in an array behind all slots' z
+// the slot's p (6 each; read in pairs, 16 consecutive slots in 32 banks).
+constexpr int kCgCache = 12;
+// Rows that a warp takes at once where a row is six lanes' work.
+constexpr int kCgLaneRows = 5;
+// What the choice of kernel counts a slot as.
+constexpr int kCgCacheAsk = 24;
 
 struct CgJob {
   int32_t model;
@@ -91,6 +105,7 @@ struct CgArgs {
   uint32_t cap_rows;        // row-state capacity (same in every CTA)
   uint32_t cap_blocks;      // cached S blocks per CTA (the rest read from global)
   uint32_t cap_slots;       // blocks per CTA whose cache slot is in shared memory
+  uint32_t cap_subs;        // subscriber entries per CTA in shared memory (0: read from global)
   const int32_t* active;
   int32_t* iters;
   int32_t max_iter;
@@ -170,9 +185,9 @@ __device__ __forceinline__ uint32_t cg_slot16(uint32_t e) {
 // Slots in shared memory, in whole 16-byte words.
 inline size_t cg_slot_bytes(uint32_t cap_slots) { return ((size_t)cap_slots * 2 + 15) / 16 * 16; }
 inline size_t cg_smem_bytes(uint32_t cap_rows, uint32_t cap_blocks, uint32_t cap_cache,
-                            uint32_t cap_slots) {
+                            uint32_t cap_slots, uint32_t cap_subs) {
   return (size_t)cap_rows * kCgRow * 4 + (size_t)cap_blocks * (36 * 4) +
-         (size_t)cap_cache * kCgCache * 4 + cg_slot_bytes(cap_slots);
+         (size_t)cap_cache * kCgCache * 4 + cg_slot_bytes(cap_slots) + (size_t)cap_subs * 4;
 }
 
 // Extra shared memory of the two-level form, in floats: per row W (42); per
@@ -223,49 +238,61 @@ __device__ __forceinline__ DFloat df_shfl_xor(DFloat v, int o) {
   return DFloat{__shfl_xor_sync(kFull, v.hi, o), __shfl_xor_sync(kFull, v.lo, o)};
 }
 
-// The cluster's totals from an inbox: lane r < cluster size (<= 16) holds CTA
-// r's values, lanes 16..31 hold zeros, and a butterfly within each half-warp
-// leaves the totals in lanes 0..15.
+// The cluster's totals from an inbox: lane r < cluster size (<= 16) of a
+// half-warp holds CTA r's values, the others zeros, and a butterfly within
+// each half-warp leaves totals in it: values 0 .. kIn - 1 in lanes 0..15, the
+// rest in lanes 16..31 (one value: in both).  The loop is rolled: this runs on
+// one warp between two barriers, where the fetch of straight-line code would
+// take longer than the sums.
 template <int N>
-__device__ __forceinline__ void cg_inbox_sum(const DFloat (*inbox)[4], int csize, int lane,
-                                             DFloat (&v)[N]) {
+struct CgInbox {
+  static constexpr int kIn = (N + 1) / 2;  // values per half-warp
+  DFloat v[kIn];
+  __device__ __forceinline__ CgInbox(const DFloat (*inbox)[4], int csize, int lane) {
+    const int r = lane & 15, first = N > 1 ? kIn * (lane >> 4) : 0;
 #pragma unroll
-  for (int i = 0; i < N; ++i) v[i] = lane < csize ? inbox[lane][i] : DFloat{0.0f, 0.0f};
+    for (int i = 0; i < kIn; ++i) v[i] = r < csize ? inbox[r][first + i] : DFloat{0.0f, 0.0f};
+#pragma unroll 1
+    for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1)
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = df_sum(v[i], df_shfl_xor(v[i], o));
-}
+      for (int i = 0; i < kIn; ++i) v[i] = df_sum(v[i], df_shfl_xor(v[i], o));
+  }
+  // Total i, in every lane.
+  __device__ __forceinline__ DFloat total(int i) const {
+    const int src = N > 1 && i >= kIn ? 16 : 0;
+    const DFloat t = v[i % kIn];
+    return DFloat{__shfl_sync(kFull, t.hi, src), __shfl_sync(kFull, t.lo, src)};
+  }
+};
 
 // Inner products: a warp sums its rows' products in FP32 (a few rows of six
 // components); the warps' partials are summed as double-floats over the CTA
-// and then over the cluster's CTAs, in a fixed order, by warp 0.  wv: N
-// (<= 4) values held by lane 0 of every warp; all threads receive the totals
-// in tot (shared memory).  Every CTA sums the same partials in the same
-// order, so every CTA sees bit-identical totals.  While warp 0 sums and
-// pushes the CTA's partials, warps 1.. run side(w) with w = warp - 1 (the
+// by warp 0, which pushes them to every CTA of the cluster, and after the
+// cluster barrier every warp sums its CTA's inbox (CgInbox): the same partials
+// in the same order everywhere, so every thread of the cluster holds
+// bit-identical totals.  wv: N (<= 4) values held by lane 0 of every warp.
+// While warp 0 sums and pushes, warps 1.. run side(w) with w = warp - 1 (the
 // coarse group sums, which read the same row state after the same CTA
-// barrier); while warp 0 sums the inbox after the cluster barrier, they run
-// after(w) (coarse work that reads what the barrier published).
+// barrier).  That every warp sums the inbox, not warp 0 for the others, saves
+// the CTA barrier after it, and the 16 warps fetch the same instructions at
+// the same time.
 //
 // Exchange by push: before the cluster barrier, lane r of warp 0 stores the
 // CTA's partials into CTA r's inbox (inbox[source rank][value]); after it,
 // every CTA reads its own inbox.  A warp that loads from many CTAs waits on
 // each remote round trip (measured: ~4.5k cycles for one load per CTA of a
 // 16-CTA cluster), while remote stores complete behind the barrier's
-// release.  Consecutive reductions use different inboxes: a CTA can only
-// write inbox n + 2 after the barrier of reduction n + 1, which every reader
+// release.  Consecutive exchanges use different inboxes: a CTA can only
+// write inbox n + 2 after the barrier of exchange n + 1, which every reader
 // of inbox n has passed.
-template <int kWarps, int N, typename Side, typename Post, typename After>
-__device__ __forceinline__ void cg_reduce(cgx::cluster_group& cl, const float (&wv)[N],
-                                          float* wsm, DFloat (*inbox)[4], DFloat* tot,
-                                          Side&& side, Post&& post, After&& after) {
+template <int kWarps, int N, typename Side>
+__device__ __forceinline__ void cg_exchange(cgx::cluster_group& cl, const float (&wv)[N],
+                                            float* wsm, DFloat (*inbox)[4], Side&& side) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0)
 #pragma unroll
     for (int i = 0; i < 4; ++i) wsm[warp * 4 + i] = i < N ? wv[i < N ? i : 0] : 0.0f;
   __syncthreads();
-  const int csize = (int)cl.num_blocks();
   if (warp == 0) {
     // lane = 4 w + i: warps w, w + 8, ... (value i) in order, then over w in
     // a fixed tree
@@ -273,14 +300,13 @@ __device__ __forceinline__ void cg_reduce(cgx::cluster_group& cl, const float (&
     DFloat c = df_sum(DFloat{wsm[lane], 0.0f}, DFloat{wsm[32 + lane], 0.0f});
 #pragma unroll
     for (int h = 2; h < kWarps / 8; ++h) c = df_sum(c, DFloat{wsm[32 * h + lane], 0.0f});
-    c = df_sum(c, df_shfl_xor(c, 4));
-    c = df_sum(c, df_shfl_xor(c, 8));
-    c = df_sum(c, df_shfl_xor(c, 16));
+#pragma unroll 1
+    for (int o = 4; o < 32; o *= 2) c = df_sum(c, df_shfl_xor(c, o));
     DFloat v[N];
 #pragma unroll
     for (int i = 0; i < N; ++i)
       v[i] = DFloat{__shfl_sync(kFull, c.hi, i), __shfl_sync(kFull, c.lo, i)};
-    if (lane < csize) {
+    if (lane < (int)cl.num_blocks()) {
       DFloat* dst = cl.map_shared_rank(&inbox[0][0], (unsigned)lane) + 4 * cl.block_rank();
 #pragma unroll
       for (int i = 0; i < N; ++i) dst[i] = v[i];
@@ -289,28 +315,7 @@ __device__ __forceinline__ void cg_reduce(cgx::cluster_group& cl, const float (&
     side(warp - 1);
   }
   cl.sync();
-  if (warp == 0) {
-    DFloat v[N];
-    cg_inbox_sum<N>(inbox, csize, lane, v);
-    if (lane == 0) {
-#pragma unroll
-      for (int i = 0; i < N; ++i) tot[i] = v[i];
-      post();  // the iteration's scalars, once per CTA
-    }
-  } else {
-    after(warp - 1);
-  }
-  __syncthreads();
 }
-
-// Scalars of the iteration, computed by thread 0 and read by every thread:
-// r.z as a double-float, b.b, α and β in FP32 (the precision of the vectors
-// they scale).
-struct CgScalars {
-  DFloat rz;
-  float b2, af, bf;
-  int stop;
-};
 
 // One output of the coarse step: sc[o] = (E^-1 w)_o for this CTA's (group,
 // mode) output o, with the model's w = W^T r − α W^T q (wq null at the
@@ -330,25 +335,6 @@ __device__ __forceinline__ void cg_coarse_dot(const float* sEi, uint32_t cap_dim
   if (lane == 0) sc[o] = v;
 }
 
-// The iteration's α as the p.q reduction's post forms it (the same sums in
-// the same order, so the same value), in every lane of the calling warp:
-// p.q from inbox 0 plus the lens row's share, α = r.z / p.q (0 where p.q
-// vanishes).
-__device__ __forceinline__ float cg_alpha(const DFloat (*inbox)[4], int csize, int lane,
-                                          int32_t lens, const float* lens_p, float rz) {
-  DFloat v[4];
-  cg_inbox_sum<4>(inbox, csize, lane, v);
-  DFloat t[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    t[i] = DFloat{__shfl_sync(kFull, v[i].hi, 0), __shfl_sync(kFull, v[i].lo, 0)};
-  DFloat pq = t[0];
-  if (lens >= 0)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) pq = df_sum(pq, df_scale(lens_p[c], t[1 + c]));
-  return fabsf(pq.hi) < 1.17549435e-38f ? 0.0f : rz / pq.hi;
-}
-
 // A row's coarse share of z, (W c)_i for lane i < 6 (rows outside every
 // group, such as the lens row, add nothing).
 __device__ __forceinline__ float cg_row_wc(const float* sWrow, int32_t lg, const float* sc,
@@ -365,21 +351,19 @@ __device__ __forceinline__ float cg_row_wc(const float* sWrow, int32_t lg, const
 // Per own group: the sum over its rows of W^T x, x the row-state vector at
 // float offset `xoff`, pushed into the model-wide array `dst` (D floats, at
 // this CTA's groups' offset) of every CTA.  A warp per (group, mode), warp
-// `w` of kWorkers taking (group, mode) w, w + kWorkers, ...: lane l takes
-// rows l, l + 32, ... (each row's six products in component order), then a
+// `w` of kWorkers taking (group, mode) w, w + kWorkers, ...: lane l takes the
+// group's rows (local rows grp[2 g] .. grp[2 g + 1]) l, l + 32, ... (each row's six products in component order), then a
 // fixed butterfly.
-__device__ __forceinline__ void cg_group_sum_push(cgx::cluster_group& cl, int o,
-                                                  const int32_t* grp_row0,
-                                                  const int32_t* grp_row1, int32_t g0,
-                                                  int32_t goff, uint32_t row0, const float* sW,
+__device__ __forceinline__ void cg_group_sum_push(cgx::cluster_group& cl, int o, const int* grp,
+                                                  int32_t goff, const float* sW,
                                                   const float* rs, int xoff, float* dst) {
   const int lane = threadIdx.x & 31;
   const int csize = (int)cl.num_blocks();
   const int l = o / kCoarseModes, j = o % kCoarseModes;
   float v = 0.0f;
-  for (int32_t r = grp_row0[g0 + l] + lane; r < grp_row1[g0 + l]; r += 32) {
-    const float* w = sW + (size_t)(r - row0) * 42 + j;
-    const float* x = rs + (size_t)(r - row0) * kCgRow + xoff;
+  for (int r = grp[2 * l] + lane; r < grp[2 * l + 1]; r += 32) {
+    const float* w = sW + (size_t)r * 42 + j;
+    const float* x = rs + (size_t)r * kCgPitch + xoff;
 #pragma unroll
     for (int i = 0; i < 6; ++i) v += w[kCoarseModes * i] * x[i];
   }
@@ -389,29 +373,32 @@ __device__ __forceinline__ void cg_group_sum_push(cgx::cluster_group& cl, int o,
 }
 template <int kWorkers>
 __device__ __forceinline__ void cg_group_sums_push(cgx::cluster_group& cl, int w, int32_t ngr,
-                                                   const int32_t* grp_row0,
-                                                   const int32_t* grp_row1, int32_t g0,
-                                                   int32_t goff, uint32_t row0, const float* sW,
+                                                   const int* grp, int32_t goff, const float* sW,
                                                    const float* rs, int xoff, float* dst) {
   for (int o = w; o < ngr * kCoarseModes; o += kWorkers)
-    cg_group_sum_push(cl, o, grp_row0, grp_row1, g0, goff, row0, sW, rs, xoff, dst);
+    cg_group_sum_push(cl, o, grp, goff, sW, rs, xoff, dst);
 }
 
-// Push a row's six values (lane i < 6 holds x_i) into the neighbour cache of
-// every CTA that reads the row, at float offset `off` of its slot there.
-__device__ __forceinline__ void cg_push_row(cgx::cluster_group& cl, float* cache,
-                                            const uint32_t* sub_ent, uint32_t s0, uint32_t s1,
-                                            float xi, int off) {
-  const int lane = threadIdx.x & 31;
-  float x[6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) x[i] = __shfl_sync(kFull, xi, i);
-  for (uint32_t t = s0 + lane; t < s1; t += 32) {
-    const uint32_t e = __ldg(sub_ent + t);
-    float* dst = cl.map_shared_rank(cache, e >> 16) + (size_t)(e & 0xffffu) * kCgCache + off;
-    *reinterpret_cast<float4*>(dst) = make_float4(x[0], x[1], x[2], x[3]);
-    *reinterpret_cast<float2*>(dst + 4) = make_float2(x[4], x[5]);
+// Push a value x of a row, its component c, into z of the neighbour cache of
+// every CTA that reads the row: its n subscribers.
+__device__ __forceinline__ void cg_push_z(cgx::cluster_group& cl, float* cz, const uint32_t* sub,
+                                          int n, float x, int c) {
+#pragma unroll 4
+  for (int t = 0; t < n; ++t) {
+    const uint32_t e = sub[t];
+    cl.map_shared_rank(cz, e >> 16)[(size_t)(e & 0xffffu) * 6 + c] = x;
   }
+}
+// A row's coarse group slot (-1: none), number of subscribers, and the first
+// of them.
+__device__ __forceinline__ int32_t cg_row_group(const float* st) {
+  return (__float_as_int(st[kCgIdx + 3]) & 7) - 1;
+}
+__device__ __forceinline__ int cg_row_nsub(const float* st) {
+  return __float_as_int(st[kCgIdx + 3]) >> 3;
+}
+__device__ __forceinline__ uint32_t cg_row_sub(const float* st) {
+  return (uint32_t)__float_as_int(st[kCgIdx + 4]);
 }
 
 // A block's 36 values from a turned run of up to 32 blocks that starts at
@@ -433,9 +420,7 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
   constexpr int kCgWarps = kThreads / 32;
   __shared__ float wsm[kCgWarps * 4];
   __shared__ DFloat inbox[3][kCgMaxCluster][4];  // reduction inboxes (push)
-  __shared__ DFloat tot[4];
   __shared__ float lens_p[4];  // the lens row's p, pushed by its owner
-  __shared__ CgScalars sc;
   __shared__ uint64_t stage_bar;  // completion of the S blocks' bulk copy
   extern __shared__ __align__(16) unsigned char cg_smem[];
   cgx::cluster_group cl = cgx::this_cluster();
@@ -449,15 +434,21 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
   const uint32_t B0 = A.row_ptr[J.row0];
   const uint32_t nblk = A.row_ptr[J.row1] - B0;
   const uint32_t ncached = nblk < A.cap_blocks ? nblk : A.cap_blocks;
+  const uint32_t sub0 = A.sub_ptr[J.row0], nsub = A.sub_ptr[J.row1] - sub0;
   const uint32_t nslots = nblk < A.cap_slots ? nblk : A.cap_slots;
   // Shared memory: row state | cached S blocks | neighbour cache | the
-  // blocks' cache slots | two-level form: W per row, E^-1 rows and c per own
+  // blocks' cache slots | the rows' subscribers | two-level form: W per row, E^-1 rows and c per own
   // group, the model's group sums of W^T r (two buffers) and W^T q.
   float* rs = reinterpret_cast<float*>(cg_smem);
+  // behind the rows, in what their pitch leaves of kCgRow: the groups' first
+  // and end local rows
+  int* sGrp = reinterpret_cast<int*>(rs + (size_t)A.cap_rows * kCgPitch);
   float* sS = rs + (size_t)A.cap_rows * kCgRow;
-  float* cache = sS + (size_t)A.cap_blocks * 36;
-  uint16_t* sL = reinterpret_cast<uint16_t*>(cache + (size_t)A.cap_cache * kCgCache);
-  float* sW = reinterpret_cast<float*>(sL + ((size_t)A.cap_slots + 7) / 8 * 8);
+  float* cz = sS + (size_t)A.cap_blocks * 36;
+  float* cp = cz + (size_t)A.cap_cache * 6;
+  uint16_t* sL = reinterpret_cast<uint16_t*>(cp + (size_t)A.cap_cache * 6);
+  uint32_t* sSub = reinterpret_cast<uint32_t*>(sL + ((size_t)A.cap_slots + 7) / 8 * 8);
+  float* sW = reinterpret_cast<float*>(sSub + A.cap_subs);
   float* sEi = sW + (size_t)A.cap_rows * 42;
   const size_t gsz = (size_t)A.cap_groups * kCoarseModes;
   float* scf = sEi + gsz * A.cap_dim;        // c, own outputs
@@ -475,17 +466,19 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
       cg_bulk_stage(&stage_bar, sS, A.S + (size_t)B0 * 36, ncached * 36u * 4u);
     for (uint32_t t = threadIdx.x; t < nslots; t += blockDim.x)
       sL[t] = (uint16_t)cg_slot16(A.blk_slot[B0 + t]);
-    // p(prev) of iteration 0 is 0 in every cached row; the z values arrive
-    // by push after the first cluster barrier.
-    for (uint32_t t = threadIdx.x; t < A.cap_cache * kCgCache; t += blockDim.x) cache[t] = 0.0f;
+    // p of the iteration before the first is 0 in every cached row; the z
+    // values arrive by push after the first cluster barrier.
+    if (A.cap_subs > 0)
+      for (uint32_t t = threadIdx.x; t < nsub; t += blockDim.x) sSub[t] = A.sub_ent[sub0 + t];
+    for (uint32_t t = threadIdx.x; t < A.cap_cache * kCgCache; t += blockDim.x) cz[t] = 0.0f;
     for (uint32_t t = threadIdx.x; t < nrows * 36; t += blockDim.x)
-      rs[(size_t)(t / 36) * kCgRow + kCgM + (t % 36)] = A.pre[36 * (size_t)J.row0 + t];
+      rs[(size_t)(t / 36) * kCgPitch + kCgM + (t % 36)] = A.pre[36 * (size_t)J.row0 + t];
     // Per row: its block range (the lens row: its diagonal block only; its
     // camera columns arrive through the camera rows' transposed terms) and
     // the position of its lens block.
     for (uint32_t lr = threadIdx.x; lr < nrows; lr += blockDim.x) {
       const uint32_t row = J.row0 + lr;
-      float* st = rs + (size_t)lr * kCgRow;
+      float* st = rs + (size_t)lr * kCgPitch;
       uint32_t b0 = A.row_ptr[row], b1 = A.row_ptr[row + 1];
       if ((int32_t)row == lens) b0 = A.diag_pos[row], b1 = b0 + 1;
       st[kCgIdx] = __int_as_float((int)b0);
@@ -495,11 +488,14 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
       if constexpr (kCoarse)
         for (int32_t l = 0; l < ngr; ++l)
           if ((int32_t)row >= A.grp_row0[cg0 + l] && (int32_t)row < A.grp_row1[cg0 + l]) lg = l;
-      st[kCgIdx + 3] = __int_as_float(lg);
-      st[kCgIdx + 4] = __int_as_float((int)A.sub_ptr[row]);
-      st[kCgIdx + 5] = __int_as_float((int)A.sub_ptr[row + 1]);
+      const uint32_t s0 = A.sub_ptr[row];
+      st[kCgIdx + 3] = __int_as_float((int)(A.sub_ptr[row + 1] - s0) * 8 + lg + 1);
+      st[kCgIdx + 4] = __int_as_float((int)(s0 - sub0));
     }
     if constexpr (kCoarse) {
+      if ((int)threadIdx.x < 2 * ngr)
+        sGrp[threadIdx.x] =
+            ((threadIdx.x & 1) ? A.grp_row1 : A.grp_row0)[cg0 + threadIdx.x / 2] - (int)J.row0;
       for (uint32_t t = threadIdx.x; t < nrows * 42; t += blockDim.x)
         sW[t] = A.W[42 * (size_t)J.row0 + t];
       const int32_t gm0 = A.model_g0[J.model];
@@ -519,7 +515,7 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
   if (ncached < nblk) {
     __syncthreads();
     for (uint32_t lr = warp; lr < nrows; lr += kCgWarps) {
-      const float* st = rs + (size_t)lr * kCgRow;
+      const float* st = rs + (size_t)lr * kCgPitch;
       const uint32_t b0 = (uint32_t)__float_as_int(st[kCgIdx]);
       const uint32_t b1 = (uint32_t)__float_as_int(st[kCgIdx + 1]);
       for (uint32_t c0 = b0; c0 < b1; c0 += 32) {
@@ -544,9 +540,14 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
   // Every CTA of the cluster has started (its shared memory is live for the
   // pushes below) and its staging is done.
   cl.sync();
+  const bool lens_here = lens >= 0 && (uint32_t)lens >= J.row0 && (uint32_t)lens < J.row1;
   const bool vl = lane < 6;
   const int ci = vl ? lane : 0;
-#define CGROW(lr) (rs + (size_t)(lr) * kCgRow)
+  // lane 6 g + c: row g and component c of kCgLaneRows rows at a time (lanes
+  // 30 and 31 repeat row 0's first components and write nothing)
+  const int gi = lane / 6, gb = gi < kCgLaneRows ? gi : 0, gc = lane - 6 * gi;
+  const uint32_t* subs = A.cap_subs > 0 ? sSub : A.sub_ent + sub0;
+#define CGROW(lr) (rs + (size_t)(lr) * kCgPitch)
   // x = 0, r = b, z = M r, p(prev) = 0 (ba.rs:164-168).  Inner products:
   // each lane accumulates its component's FP64 products over the warp's rows;
   // the lanes are summed once per phase.
@@ -567,33 +568,30 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
     }
   }
   const float w2[2] = {cg_sum8f(drz), cg_sum8f(dbb)};
+  // The iteration's scalars, in every thread: r.z, b.b and β in FP32 (the
+  // precision of the vectors they scale).
+  float rz, b2, bf = 0.0f;
   // r.z and b.b; the two-level form pushes the group sums of W^T b beside it
   // and forms c = E^-1 W^T b after the barrier (z = B^-1 b + W c below)
-  cg_reduce<kCgWarps, 2>(
-      cl, w2, wsm, inbox[1], tot,
-      [&](int w) {
-        if constexpr (kCoarse)
-          cg_group_sums_push<kCgWarps - 1>(cl, w, ngr, A.grp_row0, A.grp_row1, cg0, goff, J.row0,
-                                           sW, rs, kCgR, wall_r);
-      },
-      [&] {
-        sc.rz = tot[0];
-        sc.b2 = tot[1].hi;
-        sc.bf = 0.0f;
-        sc.stop = 0;
-      },
-      [&](int w) {
-        if constexpr (kCoarse) {
-          for (int o = w; o < nco; o += kCgWarps - 1)
-            cg_coarse_dot(sEi, A.cap_dim, cD, o, wall_r, nullptr, 0.0f, scf);
-        }
-      });
+  cg_exchange<kCgWarps, 2>(cl, w2, wsm, inbox[1], [&](int w) {
+    if constexpr (kCoarse)
+      cg_group_sums_push<kCgWarps - 1>(cl, w, ngr, sGrp, goff, sW, rs, kCgR, wall_r);
+  });
+  {
+    const CgInbox<2> in(inbox[1], (int)csz, lane);
+    rz = in.total(0).hi, b2 = in.total(1).hi;
+  }
+  if constexpr (kCoarse) {
+    for (int o = warp - 1; o >= 0 && o < nco; o += kCgWarps - 1)
+      cg_coarse_dot(sEi, A.cap_dim, cD, o, wall_r, nullptr, 0.0f, scf);
+    __syncthreads();
+  }
   if constexpr (kCoarse) {
     // z = B^-1 b + W E^-1 W^T b, and r . z with it.
     float drz0 = 0.0f;
     for (uint32_t lr = warp; lr < nrows; lr += kCgWarps) {
       float* st = CGROW(lr);
-      const int32_t lg = __float_as_int(st[kCgIdx + 3]);
+      const int32_t lg = cg_row_group(st);
       const float add = cg_row_wc(sW + (size_t)lr * 42, lg, scf, ci);
       float zi = 0.0f;
       if (vl) {
@@ -601,17 +599,15 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
         st[kCgZ + ci] = zi;
         drz0 += st[kCgR + ci] * zi;
       }
-      cg_push_row(cl, cache, A.sub_ent, (uint32_t)__float_as_int(st[kCgIdx + 4]),
-                  (uint32_t)__float_as_int(st[kCgIdx + 5]), zi, 0);
+      if (vl) cg_push_z(cl, cz, subs + cg_row_sub(st), cg_row_nsub(st), zi, ci);
     }
     const float w1[1] = {cg_sum8f(drz0)};
-    cg_reduce<kCgWarps, 1>(cl, w1, wsm, inbox[2], tot, [](int) {}, [&] { sc.rz = tot[0]; },
-                           [](int) {});
+    cg_exchange<kCgWarps, 1>(cl, w1, wsm, inbox[2], [](int) {});
+    rz = CgInbox<1>(inbox[2], (int)csz, lane).total(0).hi;
   } else {
     for (uint32_t lr = warp; lr < nrows; lr += kCgWarps) {
       const float* st = CGROW(lr);
-      cg_push_row(cl, cache, A.sub_ent, (uint32_t)__float_as_int(st[kCgIdx + 4]),
-                  (uint32_t)__float_as_int(st[kCgIdx + 5]), vl ? st[kCgZ + ci] : 0.0f, 0);
+      if (vl) cg_push_z(cl, cz, subs + cg_row_sub(st), cg_row_nsub(st), st[kCgZ + ci], ci);
     }
     cl.sync();  // z of iteration 0 in every cache
   }
@@ -619,8 +615,10 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
   const int32_t max_it = A.cap ? min(A.max_iter, A.cap[J.model]) : A.max_iter;
   for (int32_t it = 0; it < max_it; ++it) {
     const int cur = it & 1, prv = cur ^ 1;
-    const float bf = sc.bf;
-    float dpq = 0.0f, dlens = 0.0f;
+    // p = z + β p of every cached row, once: the rows' owners push z only.
+    for (uint32_t t = threadIdx.x; t < A.cap_cache * 6; t += kThreads) cp[t] = cz[t] + cp[t] * bf;
+    __syncthreads();
+    // q = S p: a lane per block of a row.
     for (uint32_t lr = warp; lr < nrows; lr += kCgWarps) {
       float* st = CGROW(lr);
       const uint32_t b0 = (uint32_t)__float_as_int(st[kCgIdx]);
@@ -629,147 +627,165 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
       for (uint32_t k = b0 + lane; k < b1; k += 32) {
         const uint32_t kk = k - B0;
         const uint32_t slot = kk < nslots ? sL[kk] : cg_slot16(__ldg(A.blk_slot + k));
-        float pp[6];
+        float m[36], pp[6];
+        if (kk < ncached)
+          load_block(sS + (size_t)kk * 36, m);
+        else
+          cg_load_turned(A.turned, k - lane, b1, lane, m);
         if (slot & kCgOwnSlot) {  // one of this CTA's rows: its row state
           const float* o = CGROW(slot & ~kCgOwnSlot);
 #pragma unroll
           for (int j = 0; j < 6; ++j) pp[j] = o[kCgZ + j] + o[kCgP + 6 * prv + j] * bf;
         } else {
-          const float* crow = cache + (size_t)slot * kCgCache;
-          const float4 z0 = *reinterpret_cast<const float4*>(crow);
-          const float4 z1 = *reinterpret_cast<const float4*>(crow + 4);
-          const float4 q0 = *reinterpret_cast<const float4*>(crow + 8 + 8 * prv);
-          const float4 q1 = *reinterpret_cast<const float4*>(crow + 8 + 8 * prv + 4);
-          pp[0] = z0.x + q0.x * bf, pp[1] = z0.y + q0.y * bf, pp[2] = z0.z + q0.z * bf;
-          pp[3] = z0.w + q0.w * bf, pp[4] = z1.x + q1.x * bf, pp[5] = z1.y + q1.y * bf;
+          const float2* pv = reinterpret_cast<const float2*>(cp + (size_t)slot * 6);
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            const float2 v = pv[j];
+            pp[2 * j] = v.x, pp[2 * j + 1] = v.y;
+          }
         }
-        float m[36];
-        if (kk < ncached)
-          load_block(sS + (size_t)kk * 36, m);
-        else
-          cg_load_turned(A.turned, k - lane, b1, lane, m);
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
-          float s = acc[i];
+          float v = acc[i];
 #pragma unroll
-          for (int j = 0; j < 6; ++j) s += m[6 * i + j] * pp[j];
-          acc[i] = s;
+          for (int j = 0; j < 6; ++j) v += m[6 * i + j] * pp[j];
+          acc[i] = v;
         }
       }
       warp_sum8(acc);  // lane 4i holds q_i
-      const float qi = __shfl_sync(kFull, acc[0], 4 * ci);
-      const float pi = st[kCgZ + ci] + st[kCgP + 6 * prv + ci] * bf;
-      __syncwarp();
-      if (vl) {
-        st[kCgQ + ci] = qi;
-        st[kCgP + 6 * cur + ci] = pi;
-      }
-      if (vl) dpq += pi * qi;
-      cg_push_row(cl, cache, A.sub_ent, (uint32_t)__float_as_int(st[kCgIdx + 4]),
-                  (uint32_t)__float_as_int(st[kCgIdx + 5]), pi, 8 + 8 * cur);
-      if ((int32_t)(J.row0 + lr) == lens) {
-        // every CTA's post needs the lens row's p (its share of p.q): push it
-        const float p0 = __shfl_sync(kFull, pi, 0), p1 = __shfl_sync(kFull, pi, 1),
-                    p2 = __shfl_sync(kFull, pi, 2);
-        if (lane < (int)cl.num_blocks()) {
-          float* dst = cl.map_shared_rank(lens_p, (unsigned)lane);
-          dst[0] = p0, dst[1] = p1, dst[2] = p2;
+      if ((lane & 3) == 0 && lane < 24) st[kCgQ + (lane >> 2)] = acc[0];
+    }
+    __syncwarp();
+    // p.q and the lens column's S_cg^T p_c, kCgLaneRows of the warp's rows at a
+    // time: lane 6 g + c has component c of row g, and lanes 0..5 add the
+    // rows' products in the rows' order.
+    float dpq = 0.0f, dlens = 0.0f;
+    for (uint32_t l0 = warp; l0 < nrows; l0 += kCgLaneRows * kCgWarps) {
+      const uint32_t lr = l0 + gi * kCgWarps;
+      const bool on = gi < kCgLaneRows && lr < nrows;
+      float* st = CGROW(on ? lr : l0);
+      const float qi = st[kCgQ + gc];
+      const float pi = st[kCgZ + gc] + st[kCgP + 6 * prv + gc] * bf;
+      if (on) st[kCgP + 6 * cur + gc] = pi;
+      const int32_t lp = on ? __float_as_int(st[kCgIdx + 2]) : -1;
+      float pt[6];
+#pragma unroll
+      for (int t = 0; t < 6; ++t) pt[t] = __shfl_sync(kFull, pi, 6 * gb + t);
+      if (lens_here) {
+        const unsigned at = __ballot_sync(kFull, on && (int32_t)(J.row0 + lr) == lens);
+        if (at) {  // every CTA needs the lens row's p (its share of p.q): push it
+          const int src = __ffs(at) - 1;
+          const float p0 = __shfl_sync(kFull, pi, src), p1 = __shfl_sync(kFull, pi, src + 1),
+                      p2 = __shfl_sync(kFull, pi, src + 2);
+          if (lane < (int)csz) {
+            float* dst = cl.map_shared_rank(lens_p, (unsigned)lane);
+            dst[0] = p0, dst[1] = p1, dst[2] = p2;
+          }
         }
       }
-      // W^T q of the row for the next coarse vector (the lens row, in no
-      // group, has W = 0; its transposed terms arrive after the reduction).
-      const int32_t lp = __float_as_int(st[kCgIdx + 2]);
-      if (lp >= 0) {  // S_cg^T p_c for the lens column
-        const int t = lane / 3, j = lane - 3 * (lane / 3);
-        const float pt = __shfl_sync(kFull, pi, t < 6 ? t : 0);
-        float v = 0.0f;
-        if (lane < 18) {
-          const uint32_t kk = (uint32_t)lp - B0;
-          const float* blk = kk < ncached ? sS + (size_t)kk * 36 : A.S + (size_t)lp * 36;
-          v = blk[6 * t + j] * pt;
+      float v = 0.0f;
+      if (lp >= 0 && gc < 3) {  // S_cg^T p_c for the lens column
+        const uint32_t kk = (uint32_t)lp - B0;
+        const float* blk = (kk < ncached ? sS + (size_t)kk * 36 : A.S + (size_t)lp * 36) + gc;
+        float w[6];
+#pragma unroll
+        for (int t = 0; t < 6; ++t) w[t] = __fmul_rn(blk[6 * t], pt[t]);
+        v = (__fadd_rn(w[0], w[1]) + __fadd_rn(w[2], w[3])) + __fadd_rn(w[4], w[5]);
+      }
+#pragma unroll
+      for (int g = 0; g < kCgLaneRows; ++g) {
+        const float pg = __shfl_sync(kFull, pi, 6 * g + ci), qg = __shfl_sync(kFull, qi, 6 * g + ci);
+        const float vg = __shfl_sync(kFull, v, 6 * g + ci);
+        const int32_t lg = __shfl_sync(kFull, lp, 6 * g);
+        if (l0 + g * kCgWarps < nrows) {
+          if (vl) dpq += pg * qg;
+          if (lg >= 0 && lane < 3) dlens += vg;  // lanes 0, 1, 2: components 0, 1, 2
         }
-        v += __shfl_down_sync(kFull, v, 3);
-        v += __shfl_down_sync(kFull, v, 6);
-        v += __shfl_down_sync(kFull, v, 12);
-        if (lane < 3) dlens += v;  // lanes 0, 1, 2: components 0, 1, 2
       }
     }
     const float w4[4] = {cg_sum8f(dpq), __shfl_sync(kFull, dlens, 0), __shfl_sync(kFull, dlens, 1),
                          __shfl_sync(kFull, dlens, 2)};
-    const bool lens_here = lens >= 0 && (uint32_t)lens >= J.row0 && (uint32_t)lens < J.row1;
     // p.q; the two-level form pushes the group sums of W^T q beside it and,
     // after the barrier, forms c = E^-1 (W^T r − α W^T q) of the next
     // residual beside warp 0
     const float* wr_cur = wall_r + (size_t)cur * A.cap_dim;
-    cg_reduce<kCgWarps, 4>(cl, w4, wsm, inbox[0], tot, [&](int w) {
+    cg_exchange<kCgWarps, 4>(cl, w4, wsm, inbox[0], [&](int w) {
       if constexpr (kCoarse)
-        cg_group_sums_push<kCgWarps - 1>(cl, w, ngr, A.grp_row0, A.grp_row1, cg0, goff, J.row0,
-                                         sW, rs, kCgQ, wall_q);
-    }, [&] {
-      DFloat pq = tot[0];
+        cg_group_sums_push<kCgWarps - 1>(cl, w, ngr, sGrp, goff, sW, rs, kCgQ, wall_q);
+    });
+    float af;
+    bool stop;
+    {
+      const CgInbox<4> in(inbox[0], (int)csz, lane);
+      DFloat pq = in.total(0);
       if (lens >= 0) {
         // The lens row's q gets the transposed camera terms; its share of
         // p.q is p_g . (sum S_cg^T p_c), with p_g pushed by its owner before
         // the barrier.
 #pragma unroll
-        for (int c = 0; c < 3; ++c) pq = df_sum(pq, df_scale(lens_p[c], tot[1 + c]));
-        if (lens_here) {
-          float* q = CGROW((uint32_t)lens - J.row0) + kCgQ;
-          for (int c = 0; c < 3; ++c) q[c] = df_sum(DFloat{q[c], 0.0f}, tot[1 + c]).hi;
+        for (int c = 0; c < 3; ++c) {
+          const DFloat t = in.total(1 + c);
+          pq = df_sum(pq, df_scale(lens_p[c], t));
+          if (lens_here && threadIdx.x == 0) {
+            float* q = CGROW((uint32_t)lens - J.row0) + kCgQ;
+            q[c] = df_sum(DFloat{q[c], 0.0f}, t).hi;
+          }
         }
       }
       // ba.rs:174 breaks on a vanishing p.q; an FP32 quotient needs it normal
-      sc.stop = fabsf(pq.hi) < 1.17549435e-38f ? 1 : 0;
-      sc.af = sc.stop ? 0.0f : sc.rz.hi / pq.hi;
-    }, [&](int w) {
-      if constexpr (kCoarse) {
-        if (w < nco) {
-          const float a = cg_alpha(inbox[0], (int)cl.num_blocks(), lane, lens, lens_p, sc.rz.hi);
-          for (int o = w; o < nco; o += kCgWarps - 1)
-            cg_coarse_dot(sEi, A.cap_dim, cD, o, wr_cur, wall_q, a, scf);
-        }
-      }
-    });
+      stop = fabsf(pq.hi) < 1.17549435e-38f;
+      af = stop ? 0.0f : rz / pq.hi;
+    }
+    if constexpr (kCoarse)
+      for (int o = warp - 1; o >= 0 && o < nco; o += kCgWarps - 1)
+        cg_coarse_dot(sEi, A.cap_dim, cD, o, wr_cur, wall_q, af, scf);
     ++spmv;
-    if (sc.stop) break;
-    const float af = sc.af;
+    if (stop) break;
+    if (kCoarse || lens_here) __syncthreads();  // c and the lens row's q
     float drr = 0.0f, drz2 = 0.0f;
-    for (uint32_t lr = warp; lr < nrows; lr += kCgWarps) {
-      float* st = CGROW(lr);
-      float ri = 0.0f;
-      if (vl) {
-        st[kCgX + ci] += st[kCgP + 6 * cur + ci] * af;
-        ri = st[kCgR + ci] - st[kCgQ + ci] * af;
-        st[kCgR + ci] = ri;
-      }
+    for (uint32_t l0 = warp; l0 < nrows; l0 += kCgLaneRows * kCgWarps) {
+      const uint32_t lr = l0 + gi * kCgWarps;
+      const bool on = gi < kCgLaneRows && lr < nrows;
+      float* st = CGROW(on ? lr : l0);
+      const float xi = st[kCgX + gc] + st[kCgP + 6 * cur + gc] * af;
+      const float ri = st[kCgR + gc] - st[kCgQ + gc] * af;
       float zi = 0.0f;
 #pragma unroll
-      for (int j = 0; j < 6; ++j) zi += st[kCgM + 6 * ci + j] * __shfl_sync(kFull, ri, j);
+      for (int j = 0; j < 6; ++j) zi += st[kCgM + 6 * gc + j] * __shfl_sync(kFull, ri, 6 * gb + j);
       if constexpr (kCoarse) {
         // z = B^-1 r + W c
-        zi += cg_row_wc(sW + (size_t)lr * 42, __float_as_int(st[kCgIdx + 3]), scf, ci);
+        zi += cg_row_wc(sW + (size_t)(on ? lr : l0) * 42, cg_row_group(st), scf, gc);
       }
-      if (vl) {
-        st[kCgZ + ci] = zi;
-        drr += ri * ri;
-        drz2 += ri * zi;
+      if (on) {
+        st[kCgX + gc] = xi;
+        st[kCgR + gc] = ri;
+        st[kCgZ + gc] = zi;
+        cg_push_z(cl, cz, subs + cg_row_sub(st), cg_row_nsub(st), zi, gc);
       }
-      cg_push_row(cl, cache, A.sub_ent, (uint32_t)__float_as_int(st[kCgIdx + 4]),
-                  (uint32_t)__float_as_int(st[kCgIdx + 5]), zi, 0);
+#pragma unroll
+      for (int g = 0; g < kCgLaneRows; ++g) {
+        const float rg = __shfl_sync(kFull, ri, 6 * g + ci), zg = __shfl_sync(kFull, zi, 6 * g + ci);
+        if (vl && l0 + g * kCgWarps < nrows) {
+          drr += rg * rg;
+          drz2 += rg * zg;
+        }
+      }
     }
     const float w2b[2] = {cg_sum8f(drr), cg_sum8f(drz2)};
     // r.r and r.z; the two-level form pushes the group sums of the next
     // W^T r beside them
-    cg_reduce<kCgWarps, 2>(cl, w2b, wsm, inbox[1], tot, [&](int w) {
+    cg_exchange<kCgWarps, 2>(cl, w2b, wsm, inbox[1], [&](int w) {
       if constexpr (kCoarse)
-        cg_group_sums_push<kCgWarps - 1>(cl, w, ngr, A.grp_row0, A.grp_row1, cg0, goff, J.row0,
-                                         sW, rs, kCgR, wall_r + (size_t)prv * A.cap_dim);
-    }, [&] {
-      sc.stop = tot[0].hi < (float)A.tol * sc.b2 ? 1 : 0;  // ba.rs:182
-      sc.bf = tot[1].hi / sc.rz.hi;                        // ba.rs:189-190
-      sc.rz = tot[1];
-    }, [](int) {});
-    if (sc.stop) break;
+        cg_group_sums_push<kCgWarps - 1>(cl, w, ngr, sGrp, goff, sW, rs, kCgR,
+                                         wall_r + (size_t)prv * A.cap_dim);
+    });
+    {
+      const CgInbox<2> in(inbox[1], (int)csz, lane);
+      const float rr = in.total(0).hi, rz1 = in.total(1).hi;
+      bf = rz1 / rz;  // ba.rs:189-190
+      rz = rz1;
+      if (rr < (float)A.tol * b2) break;  // ba.rs:182
+    }
   }
   for (uint32_t lr = warp; lr < nrows; lr += kCgWarps)
     if (vl) A.x[6 * (size_t)(J.row0 + lr) + ci] = CGROW(lr)[kCgX + ci];

@@ -186,6 +186,7 @@ inline bool plan_cluster(const Context& ctx, const std::vector<uint32_t>& row_pt
 struct CachePlan {
   std::vector<uint32_t> blk_slot, sub_ptr, sub_ent;
   uint32_t cap = 0;
+  uint32_t subs = 0;  // most subscribers of a CTA's rows
 };
 
 inline bool plan_cache(const ClusterPlan& cp, int csize, const std::vector<uint32_t>& row_ptr,
@@ -228,6 +229,8 @@ inline bool plan_cache(const ClusterPlan& cp, int csize, const std::vector<uint3
   pl.sub_ent.reserve(std::max<size_t>(pl.sub_ptr[nb], 1));
   for (int64_t r = 0; r < nb; ++r) pl.sub_ent.insert(pl.sub_ent.end(), subs[r].begin(), subs[r].end());
   if (pl.sub_ent.empty()) pl.sub_ent.push_back(0);
+  for (const CgJob& J : cp.jobs)
+    pl.subs = std::max(pl.subs, pl.sub_ptr[J.row1] - pl.sub_ptr[J.row0]);
   return true;
 }
 
@@ -989,7 +992,10 @@ struct LmEngine {
     const detail::CgKernel kfn = detail::cg_kernel(coarse, threads, false);
     cudaFuncAttributes fa{};
     check(cudaFuncGetAttributes(&fa, kfn), "func attr");
-    const size_t avail = (size_t)smem_optin - fa.sharedSizeBytes;
+    // (the static arrays are counted as no less than when the choices below
+    // were measured)
+    const size_t avail =
+        (size_t)smem_optin - std::max(fa.sharedSizeBytes, (size_t)(1616 + threads / 2));
     // Row state takes at most half of the shared memory (the rest caches S
     // blocks); with the coarse correction, which needs far fewer PCG
     // iterations, rows may take all of it and S is read from L2.
@@ -1027,19 +1033,19 @@ struct LmEngine {
     if (!detail::plan_cache(cp, csize, SB.h_row_ptr, h_col_idx, h_diag_pos, h_lens, ctx.nb, true,
                             kp))
       return unusable("a CTA's neighbour cache exceeds 65,535 rows");
-    if (row_bytes + coarse_bytes + (size_t)kp.cap * kCgCache * 4 +
+    if (row_bytes + coarse_bytes + (size_t)kp.cap * kCgCacheAsk * 4 +
             (size_t)(cp.max_blocks / 4 + 1) * (36 * 4 + 4) >= avail &&
         !detail::plan_cache(cp, csize, SB.h_row_ptr, h_col_idx, h_diag_pos, h_lens, ctx.nb, false,
                             kp))
       return unusable("a CTA's neighbour cache exceeds 65,535 rows");
-    const size_t cache_bytes = (size_t)kp.cap * kCgCache * 4;
+    const size_t cache_bytes = (size_t)kp.cap * kCgCacheAsk * 4;
     if (row_bytes + coarse_bytes + cache_bytes >= avail)
       return unusable("row state and neighbour cache do not fit");
-    const size_t fixed_bytes = row_bytes + coarse_bytes + cache_bytes;
     // Whether the clusters serve: with every S block cached that fits beside a
     // slot of 4 bytes each.
-    size_t smem = fixed_bytes +
-                  std::min<size_t>(cp.max_blocks, (avail - fixed_bytes) / (36 * 4 + 4)) * (36 * 4 + 4);
+    const size_t ask_bytes = row_bytes + coarse_bytes + cache_bytes;
+    size_t smem = ask_bytes +
+                  std::min<size_t>(cp.max_blocks, (avail - ask_bytes) / (36 * 4 + 4)) * (36 * 4 + 4);
     check(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)avail),
           "cluster smem");
     if (csize > 8)
@@ -1069,14 +1075,18 @@ struct LmEngine {
     // resident at once (one wave); otherwise models would queue behind each
     // other while the grid kernel runs them all together.
     if (!required && !prefer_cluster && (int64_t)nclusters < ctx.nm) return false;
-    // What a CTA keeps within `bytes` of shared memory: the cache slots of its
-    // blocks (2 bytes each), then S blocks.
-    uint32_t cap_slots = 0, cap_blocks = 0;
+    // What a CTA keeps within `bytes` of shared memory: the subscribers of its
+    // rows, the cache slots of its blocks (2 bytes each), then S blocks.
+    const size_t fixed_bytes = row_bytes + coarse_bytes + (size_t)kp.cap * kCgCache * 4;
+    uint32_t cap_subs = 0, cap_slots = 0, cap_blocks = 0;
     auto fill = [&](size_t bytes) {
-      cap_slots = (uint32_t)std::min<size_t>(cp.need_blocks, (bytes - fixed_bytes) / 16 * 8);
-      cap_blocks = (uint32_t)std::min<size_t>(
-          cp.need_blocks, (bytes - fixed_bytes - cg_slot_bytes(cap_slots)) / (36 * 4));
-      return cg_smem_bytes(cp.max_rows, cap_blocks, kp.cap, cap_slots) + coarse_bytes;
+      size_t left = bytes - fixed_bytes;
+      cap_subs = kp.subs * 4 <= left ? kp.subs : 0;
+      left -= cap_subs * 4;
+      cap_slots = (uint32_t)std::min<size_t>(cp.need_blocks, left / 16 * 8);
+      left -= cg_slot_bytes(cap_slots);
+      cap_blocks = (uint32_t)std::min<size_t>(cp.need_blocks, left / (36 * 4));
+      return cg_smem_bytes(cp.max_rows, cap_blocks, kp.cap, cap_slots, cap_subs) + coarse_bytes;
     };
     smem = fill(avail);
     // More models than clusters at a time: two CTAs an SM, each with the S
@@ -1091,7 +1101,7 @@ struct LmEngine {
             "attr");
       const detail::CgKernel kf2 = detail::cg_kernel(coarse, threads, true);
       const size_t half = ((size_t)per_sm / 2 - (size_t)reserved - fa.sharedSizeBytes) / 16 * 16;
-      if (half < smem && fixed_bytes + cg_slot_bytes(cp.need_blocks) <= half) {
+      if (half < smem && fixed_bytes + kp.subs * 4 + cg_slot_bytes(cp.need_blocks) <= half) {
         check(cudaFuncSetAttribute(kf2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)half),
               "cluster smem");
         if (csize > 8)
@@ -1111,7 +1121,7 @@ struct LmEngine {
     detail::h2d(cg_sube, kp.sub_ent, s);
     ca = CgArgs{cg_jobs, cg_loc, SB.row_ptr, SB.col_idx, (const float*)S.p, (const float*)pre.p,
                 (const float*)g.p, (float*)x.p, lens_row, lens_pos, SB.diag_pos, cp.max_rows,
-                cap_blocks, cap_slots, active, pcg_iters, pcg_limit, o.pcg_tol};
+                cap_blocks, cap_slots, cap_subs, active, pcg_iters, pcg_limit, o.pcg_tol};
     ca.order = cg_order;
     ca.cap = pcg_cap;
     ca.blk_slot = cg_slot, ca.sub_ptr = cg_subp, ca.sub_ent = cg_sube, ca.cap_cache = kp.cap;
