@@ -141,9 +141,11 @@ uint64_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n,
 void radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp,
                         uint32_t* vals_tmp, size_t n, int bits,
                         cudaStream_t s);
-void radix_sort_u64_u64(uint64_t* keys, uint64_t* vals, uint64_t* keys_tmp,
-                        uint64_t* vals_tmp, size_t n, int bits,
-                        cudaStream_t s);
+// The same with buffers of equal size: the sorted arrays are left in `keys`
+// and `vals`, which may have changed places with the *_tmp buffers.
+void radix_sort_u64_u64(DevBuf<uint64_t>& keys, DevBuf<uint64_t>& vals,
+                        DevBuf<uint64_t>& keys_tmp, DevBuf<uint64_t>& vals_tmp, size_t n,
+                        int bits, cudaStream_t s);
 
 // p[i] = lower_bound(sorted[0..n), i) for i in [0, m].
 void lower_bounds_u32(const uint32_t* sorted, size_t n, uint32_t* p, size_t m,
