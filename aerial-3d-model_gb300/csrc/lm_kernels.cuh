@@ -1297,78 +1297,109 @@ static __global__ void __launch_bounds__(FusedPoint<kChunk>::kThreads,
 // ---- per camera: U, g, lens terms (ba.rs:273-292) ----------------------------
 
 constexpr int kCamThreads = 128;
-constexpr int kCamN = 45;  // 21 U | 18 X | 6 lens U     (storage precision)
-constexpr int kCamG = 18;  // 6 gj | 6 gs | 3 lg | 3 ls  (FP64)
+constexpr int kCamN = 45;  // 21 U | 18 X | 6 lens U
 
-// FP64 form, per camera (ba.rs:273-292): every sum in FP64; a CTA per camera,
-// its observations gathered through the camera ordering.  (The mixed form
-// runs camera_mixed_kernel.)
-template <typename R>
-__global__ void __launch_bounds__(kCamThreads)
-    camera_kernel(Prob P, StructView S, IterBufs<R> B, const int32_t* active) {
-  static_assert(sizeof(R) == 8, "the mixed form runs camera_mixed_kernel");
-  __shared__ double scratch[kCamN * 32];
-  __shared__ double gscratch[kCamG * 32];
-  const int64_t c = blockIdx.x;
-  if (c >= P.nc) return;
-  const uint32_t m = P.cam_model[c];
-  if (!active[m]) return;
-  const bool refine = P.model_refine[m] != 0;
-  double accd[kCamN];
-  double gacc[kCamG];
+// FP64 form, per camera (ba.rs:273-292): every sum in FP64.  All products are
+// w (r0_p r0_q + r1_p r1_q) of the observation's two rows r = (Jc | Jg | e):
+// entries 0..5, 6..8 and 9.  A camera's 63 sums are shared out to kCamUnits
+// CTAs of about 21 operations an observation each (7 products; 6 and the
+// plain sums of the gradient shares), which gather its observations through
+// the camera ordering.  Bound by the FP64 operations, 64 cycles of an SM
+// sub-partition each: a CTA per camera left most SMs idle below 152 cameras
+// and filled them unevenly above (500 cameras: 4 on some, 3 on others, at 188
+// registers).  500 cameras with 2.6 M observations: 1142 -> 1022 us; 77 with
+// 0.26 M: 268 -> 136.
+constexpr int kCamUnits = 8;
+struct CamPair {
+  int p, q;
+};
+template <int U>
+struct CamUnit {
+  static constexpr bool kRefine = U >= 3 && U <= 6;  // of a model that refines its lens only
+  static constexpr int kPairs = U < 6 ? 7 : 6;
+  static constexpr int kAdds = U == 6 ? 3 : U == 7 ? 6 : 0;  // sums of gsub
+  static constexpr int kAdd0 = U == 6 ? 6 : 0;               // from gsub[kAdd0]
+  static __host__ __device__ constexpr CamPair pair(int i) {
+    if (U == 0) return i < 6 ? CamPair{0, i} : CamPair{5, 5};
+    if (U == 1) return i < 5 ? CamPair{1, 1 + i} : CamPair{4, i - 1};
+    if (U == 2) return i < 4 ? CamPair{2, 2 + i} : CamPair{3, i - 1};
+    if (U < 6) return i < 6 ? CamPair{2 * (U - 3) + i / 3, 6 + i % 3} : CamPair{U + 3, 9};
+    if (U == 6) return i < 3 ? CamPair{6, 6 + i} : i < 5 ? CamPair{7, 4 + i} : CamPair{8, 8};
+    return CamPair{i, 9};
+  }
+  // whether an entry of the rows is in one of the pairs
+  static __host__ __device__ constexpr bool reads(int e) {
+    for (int i = 0; i < kPairs; ++i)
+      if (pair(i).p == e || pair(i).q == e) return true;
+    return false;
+  }
+};
+
+template <int U, typename R>
+__device__ __forceinline__ void camera_unit(const Prob& P, const StructView& S,
+                                            const IterBufs<R>& B, int64_t c, double* scratch) {
+  using Un = CamUnit<U>;
+  constexpr int kN = Un::kPairs + Un::kAdds;
+  double acc[kN];
 #pragma unroll
-  for (int i = 0; i < kCamN; ++i) accd[i] = 0.0;
-#pragma unroll
-  for (int i = 0; i < kCamG; ++i) gacc[i] = 0.0;
+  for (int i = 0; i < kN; ++i) acc[i] = 0.0;
   const uint32_t b = S.cam_ptr[c], e = S.cam_ptr[c + 1];
-  for (uint32_t i = b + threadIdx.x; i < e; i += blockDim.x) {
+  const bool on = !Un::kRefine || P.model_refine[P.cam_model[c]] != 0;
+  for (uint32_t i = on ? b + threadIdx.x : e; i < e; i += kCamThreads) {
     const uint32_t k = S.cam_obs[i];
     const double* o = B.lin + (size_t)k * kLinW;
     if (o[27] == 0.0 || !B.kept[P.obs_pt[k]]) continue;  // ba.rs:274-277
     const double w = o[26];
-    double jc[12];
+    double r0[10], r1[10];
 #pragma unroll
-    for (int t = 0; t < 12; ++t) jc[t] = o[t];
-    int u = 0;
-#pragma unroll
-    for (int a = 0; a < 6; ++a)
-#pragma unroll
-      for (int bb = a; bb < 6; ++bb) accd[u++] += (jc[a] * jc[bb] + jc[6 + a] * jc[6 + bb]) * w;
-    const double* gs = B.gsub + (size_t)k * 9;
-    const double e0 = o[24], e1 = o[25];
-#pragma unroll
-    for (int a = 0; a < 6; ++a) {
-      gacc[a] += (jc[a] * e0 + jc[6 + a] * e1) * w;
-      gacc[6 + a] += gs[a];
-    }
-    if (refine) {
-      const double jg[6] = {o[18], o[19], o[20], o[21], o[22], o[23]};
-#pragma unroll
-      for (int a = 0; a < 6; ++a)
-#pragma unroll
-        for (int bb = 0; bb < 3; ++bb)
-          accd[21 + 3 * a + bb] += (jc[a] * jg[bb] + jc[6 + a] * jg[3 + bb]) * w;
-      int v = 0;
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int bb = a; bb < 3; ++bb) accd[39 + v++] += (jg[a] * jg[bb] + jg[3 + a] * jg[3 + bb]) * w;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        gacc[12 + a] += (jg[a] * e0 + jg[3 + a] * e1) * w;
-        gacc[15 + a] += gs[6 + a];
+    for (int t = 0; t < 10; ++t)
+      if (Un::reads(t)) {
+        r0[t] = o[t < 6 ? t : t < 9 ? 12 + t : 24];
+        r1[t] = o[t < 6 ? 6 + t : t < 9 ? 15 + t : 25];
       }
+#pragma unroll
+    for (int t = 0; t < Un::kPairs; ++t) {
+      const CamPair q = Un::pair(t);
+      acc[t] += (r0[q.p] * r0[q.q] + r1[q.p] * r1[q.q]) * w;
     }
+#pragma unroll
+    for (int t = 0; t < Un::kAdds; ++t)
+      acc[Un::kPairs + t] += B.gsub[(size_t)k * 9 + Un::kAdd0 + t];
   }
-  block_sum<kCamN>(accd, scratch);
-  block_sum<kCamG>(gacc, gscratch);
+  block_sum<kN>(acc, scratch);
   if (threadIdx.x == 0) {
-    double* U = B.camU + 21 * c;
-    for (int i = 0; i < 21; ++i) U[i] = accd[i];
-    for (int i = 0; i < 6; ++i) B.camgj[6 * c + i] = gacc[i], B.camgs[6 * c + i] = gacc[6 + i];
-    for (int i = 0; i < 18; ++i) B.camX[18 * c + i] = accd[21 + i];
-    for (int i = 0; i < 6; ++i) B.caml[12 * c + i] = accd[39 + i];
-    for (int i = 0; i < 6; ++i) B.caml[12 * c + 6 + i] = gacc[12 + i];
+#pragma unroll
+    for (int t = 0; t < Un::kPairs; ++t) {
+      const int p = Un::pair(t).p, q = Un::pair(t).q;
+      if (q < 6) B.camU[21 * c + 6 * p - p * (p - 1) / 2 + (q - p)] = acc[t];
+      else if (p < 6 && q < 9) B.camX[18 * c + 3 * p + (q - 6)] = acc[t];
+      else if (p < 6) B.camgj[6 * c + p] = acc[t];
+      else if (q < 9) B.caml[12 * c + 3 * (p - 6) - (p - 6) * (p - 7) / 2 + (q - p)] = acc[t];
+      else B.caml[12 * c + p] = acc[t];
+    }
+#pragma unroll
+    for (int t = 0; t < Un::kAdds; ++t)
+      if (U == 7) B.camgs[6 * c + t] = acc[Un::kPairs + t];
+      else B.caml[12 * c + 9 + t] = acc[Un::kPairs + t];
+  }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kCamThreads)
+    camera_kernel(Prob P, StructView S, IterBufs<R> B, const int32_t* active) {
+  static_assert(sizeof(R) == 8, "the mixed form runs camera_mixed_kernel");
+  __shared__ double scratch[12 * 32];
+  const int64_t c = blockIdx.x / kCamUnits;
+  if (c >= P.nc || !active[P.cam_model[c]]) return;
+  switch (blockIdx.x % kCamUnits) {
+    case 0: return camera_unit<0>(P, S, B, c, scratch);
+    case 1: return camera_unit<1>(P, S, B, c, scratch);
+    case 2: return camera_unit<2>(P, S, B, c, scratch);
+    case 3: return camera_unit<3>(P, S, B, c, scratch);
+    case 4: return camera_unit<4>(P, S, B, c, scratch);
+    case 5: return camera_unit<5>(P, S, B, c, scratch);
+    case 6: return camera_unit<6>(P, S, B, c, scratch);
+    default: return camera_unit<7>(P, S, B, c, scratch);
   }
 }
 

@@ -1384,7 +1384,8 @@ struct LmEngine {
         BA_LAUNCH(camera_mixed_kernel<<<(unsigned)ctx.nc, kCamMixThreads, 0, cs>>>(P, SV, B,
                                                                                   active));
       else
-        BA_LAUNCH(camera_kernel<R><<<(unsigned)ctx.nc, kCamThreads, 0, cs>>>(P, SV, B, active));
+        BA_LAUNCH(camera_kernel<R><<<(unsigned)(ctx.nc * kCamUnits), kCamThreads, 0, cs>>>(
+            P, SV, B, active));
     }
     BA_LAUNCH(group_kernel<<<grid_for(ctx.ng * 32, 128), 128, 0, cs>>>(P, SV, caml, grpU, grpg,
                                                                       active));
