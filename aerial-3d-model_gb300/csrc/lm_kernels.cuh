@@ -4,6 +4,7 @@
 // the 3x3 / 6x6 block inversions are always FP64.
 #pragma once
 
+#include "mul_int.cuh"
 #include "solver.cuh"
 #include "structure.cuh"
 
@@ -1307,8 +1308,8 @@ constexpr int kCamN = 45;  // 21 U | 18 X | 6 lens U
 // the camera ordering.  Bound by the FP64 operations, 64 cycles of an SM
 // sub-partition each: a CTA per camera left most SMs idle below 152 cameras
 // and filled them unevenly above (500 cameras: 4 on some, 3 on others, at 188
-// registers).  500 cameras with 2.6 M observations: 1142 -> 1022 us; 77 with
-// 0.26 M: 268 -> 136.
+// registers).  500 cameras with 2.6 M observations: 1142 -> 866 us (1022 with all operations on the FP64 pipe); 77 with
+// 0.26 M: 268 -> 122.
 constexpr int kCamUnits = 8;
 struct CamPair {
   int p, q;
@@ -1351,16 +1352,31 @@ __device__ __forceinline__ void camera_unit(const Prob& P, const StructView& S,
     if (o[27] == 0.0 || !B.kept[P.obs_pt[k]]) continue;  // ba.rs:274-277
     const double w = o[26];
     double r0[10], r1[10];
+    bool safe = true;
 #pragma unroll
     for (int t = 0; t < 10; ++t)
       if (Un::reads(t)) {
         r0[t] = o[t < 6 ? t : t < 9 ? 12 + t : 24];
         r1[t] = o[t < 6 ? 6 + t : t < 9 ? 15 + t : 25];
+        safe = safe && mul_safe(r1[t]);
       }
+    // of a pair's three operations the product r1_p r1_q in integers
+    if (safe) {
+      MulOp m[10];
 #pragma unroll
-    for (int t = 0; t < Un::kPairs; ++t) {
-      const CamPair q = Un::pair(t);
-      acc[t] += (r0[q.p] * r0[q.q] + r1[q.p] * r1[q.q]) * w;
+      for (int t = 0; t < 10; ++t)
+        if (Un::reads(t)) m[t] = mul_op(r1[t]);
+#pragma unroll
+      for (int t = 0; t < Un::kPairs; ++t) {
+        const CamPair q = Un::pair(t);
+        acc[t] = fma(fma(r0[q.p], r0[q.q], mul_int(m[q.p], m[q.q])), w, acc[t]);
+      }
+    } else {
+#pragma unroll
+      for (int t = 0; t < Un::kPairs; ++t) {
+        const CamPair q = Un::pair(t);
+        acc[t] = fma(fma(r0[q.p], r0[q.q], __dmul_rn(r1[q.p], r1[q.q])), w, acc[t]);
+      }
     }
 #pragma unroll
     for (int t = 0; t < Un::kAdds; ++t)
@@ -1963,12 +1979,44 @@ __device__ __forceinline__ void schur_segment(const Prob& P, const StructView& S
       load_Zl(B, (size_t)(eb - P.no), zb);
     }
     int n = 0;
+    if constexpr (sizeof(R) == 8) {
+      // An entry takes a product, two fused ones and the addition to the sum,
+      // four operations of the FP64 pipe; where the factors allow it the first
+      // is made in integers.
+      bool safe = true;
 #pragma unroll
-    for (int r = 0; r < O::kRows; ++r)
+      for (int r = 0; r < O::kRows; ++r) safe = safe && mul_safe(za[3 * r + 1]);
+      if constexpr (!O::kSym)
 #pragma unroll
-      for (int c = O::kSym ? r : 0; c < O::kCols; ++c)
-        acc[n++] += za[3 * r] * zb[3 * c] + za[3 * r + 1] * zb[3 * c + 1] +
-                    za[3 * r + 2] * zb[3 * c + 2];
+        for (int c = 0; c < O::kCols; ++c) safe = safe && mul_safe(zb[3 * c + 1]);
+      if (safe) {
+        MulOp mb[O::kCols];
+#pragma unroll
+        for (int c = 0; c < O::kCols; ++c) mb[c] = mul_op(zb[3 * c + 1]);
+#pragma unroll
+        for (int r = 0; r < O::kRows; ++r) {
+          const MulOp ma = mul_op(za[3 * r + 1]);
+#pragma unroll
+          for (int c = O::kSym ? r : 0; c < O::kCols; ++c)
+            acc[n++] += fma(za[3 * r + 2], zb[3 * c + 2],
+                            fma(za[3 * r], zb[3 * c], mul_int(ma, mb[c])));
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < O::kRows; ++r)
+#pragma unroll
+          for (int c = O::kSym ? r : 0; c < O::kCols; ++c)
+            acc[n++] += fma(za[3 * r + 2], zb[3 * c + 2],
+                            fma(za[3 * r], zb[3 * c], __dmul_rn(za[3 * r + 1], zb[3 * c + 1])));
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < O::kRows; ++r)
+#pragma unroll
+        for (int c = O::kSym ? r : 0; c < O::kCols; ++c)
+          acc[n++] += za[3 * r] * zb[3 * c] + za[3 * r + 1] * zb[3 * c + 1] +
+                      za[3 * r + 2] * zb[3 * c + 2];
+    }
   }
   int off = 0, cnt = O::kN;
   R v[2];
@@ -1995,7 +2043,8 @@ __device__ __forceinline__ void schur_segment(const Prob& P, const StructView& S
 // Warp per sub-segment.  FP64 form: bound by its operations, of which the
 // kinds leave out what is zero or a mirror image (a sixth of them on the
 // 500-camera survey: 17 % of the pairs are an observation with itself, 20 % end
-// in a lens entry); 128 threads, three CTAs of 166 registers a thread.  FP32
+// in a lens entry; 57.2 -> 45.7 ms a solve) and a quarter is made in integers
+// (45.7 -> 34.4 ms); 128 threads, three CTAs of 168 registers a thread.  FP32
 // form: bound by the latency of its gathers (three CTAs of 256 threads, 80
 // registers); an observation with itself is gathered once, a lens entry with
 // three loads.
