@@ -200,6 +200,33 @@ __device__ __forceinline__ void chol3(const double* A, double* L) {
 
 // ---- per point: linearise its observations, V, v, V^-1, Z (ba.rs:222-268) ----
 
+// a b + c d as the compiler fuses it: the second product is rounded.
+__device__ __forceinline__ double sum2(double a, double b, double c, double d) {
+  return fma(a, b, mul_any(c, d));
+}
+
+// Two neighbouring values of a record on a 16-byte boundary.
+__device__ __forceinline__ double2 load2(const double* p) {
+  return *reinterpret_cast<const double2*>(p);
+}
+__device__ __forceinline__ void store2(double* p, double a, double b) {
+  *reinterpret_cast<double2*>(p) = make_double2(a, b);
+}
+// A record of kLinW values (a multiple of 32 bytes on such a boundary).
+__device__ __forceinline__ void store_lin(double* p, const double (&o)[kLinW]) {
+  static_assert(kLinW % 4 == 0, "whole 32-byte stores");
+#pragma unroll
+  for (int i = 0; i < kLinW; i += 4)
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p + i), "d"(o[i]), "d"(o[i + 1]),
+                 "d"(o[i + 2]), "d"(o[i + 3])
+                 : "memory");
+}
+
+// A point's records lie apart from its neighbours' in the warp, so every
+// access of a lane is a sector of its own: they move in 16- and 32-byte
+// pieces, and the point's first lens entry is summed with V.  (2.6 M
+// observations, 400 k points: 1.87 -> 1.35 ms, of which the products in integers
+// 0.18.)
 template <typename R>
 __device__ __forceinline__ void point_system(const Prob& P, const StateView& st,
                                              const StructView& S, const IterBufs<R>& B,
@@ -221,24 +248,39 @@ __device__ __forceinline__ void point_system(const Prob& P, const StateView& st,
   // V, v and the Y / Z products accumulate in the storage precision R; the 3x3
   // inversion and its Cholesky factor are FP64.
   R V[6] = {0, 0, 0, 0, 0, 0}, v[3] = {0, 0, 0};
+  // Y_g = sum over the point's observations in group g (ba.rs:251-259), of the
+  // first lens entry
+  R Y[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  const uint32_t l0 = S.lens_ptr[p], l1 = S.lens_ptr[p + 1];
   for (uint32_t k = s; k < e; ++k) {
-    R* o = B.lin + (size_t)k * kLinW;
-    if (!linearise<R>(P, st, k, sg, refine, o)) {
+    R o[kLinW];
+    const bool front = linearise<R>(P, st, k, sg, refine, o);
+    if (!front)
+#pragma unroll
       for (int i = 0; i < kLinW; ++i) o[i] = (R)0;
-      continue;
-    }
+    store_lin(B.lin + (size_t)k * kLinW, o);
+    if (!front) continue;
     const R w = o[26];
     const R j0 = o[12], j1 = o[13], j2 = o[14], j3 = o[15], j4 = o[16], j5 = o[17];
     const R e0 = o[24], e1 = o[25];
-    V[0] += (j0 * j0 + j3 * j3) * w;
-    V[1] += (j0 * j1 + j3 * j4) * w;
-    V[2] += (j0 * j2 + j3 * j5) * w;
-    V[3] += (j1 * j1 + j4 * j4) * w;
-    V[4] += (j1 * j2 + j4 * j5) * w;
-    V[5] += (j2 * j2 + j5 * j5) * w;
-    v[0] += (j0 * e0 + j3 * e1) * w;
-    v[1] += (j1 * e0 + j4 * e1) * w;
-    v[2] += (j2 * e0 + j5 * e1) * w;
+    V[0] = fma(sum2(j0, j0, j3, j3), w, V[0]);
+    V[1] = fma(sum2(j0, j1, j3, j4), w, V[1]);
+    V[2] = fma(sum2(j0, j2, j3, j5), w, V[2]);
+    V[3] = fma(sum2(j1, j1, j4, j4), w, V[3]);
+    V[4] = fma(sum2(j1, j2, j4, j5), w, V[4]);
+    V[5] = fma(sum2(j2, j2, j5, j5), w, V[5]);
+    v[0] = fma(sum2(j0, e0, j3, e1), w, v[0]);
+    v[1] = fma(sum2(j1, e0, j4, e1), w, v[1]);
+    v[2] = fma(sum2(j2, e0, j5, e1), w, v[2]);
+    if (l1 > l0 && S.obs_lens[k] == l0) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const R ga = o[18 + a], gb = o[21 + a];
+        Y[3 * a + 0] = fma(sum2(ga, j0, gb, j3), w, Y[3 * a + 0]);
+        Y[3 * a + 1] = fma(sum2(ga, j1, gb, j4), w, Y[3 * a + 1]);
+        Y[3 * a + 2] = fma(sum2(ga, j2, gb, j5), w, Y[3 * a + 2]);
+      }
+    }
   }
   double A[9], Ai[9], Vd[6];
 #pragma unroll
@@ -266,37 +308,47 @@ __device__ __forceinline__ void point_system(const Prob& P, const StateView& st,
     const R* o = B.lin + (size_t)k * kLinW;
     R* Z = B.Z + (size_t)k * 18;
     R* gs = B.gsub + (size_t)k * 9;
-    if (!ok || o[27] == (R)0) {
+    const double2 wv = load2(o + 26);  // w, valid
+    if (!ok || wv.y == 0.0) {
 #pragma unroll
       for (int i = 0; i < 18; ++i) Z[i] = (R)0;
 #pragma unroll
       for (int i = 0; i < 9; ++i) gs[i] = (R)0;
       continue;
     }
-    const R w = o[26];
-    const R j0 = o[12], j1 = o[13], j2 = o[14], j3 = o[15], j4 = o[16], j5 = o[17];
+    const R w = wv.x;
+    const double2 j01 = load2(o + 12), j23 = load2(o + 14), j45 = load2(o + 16);
+    const R j0 = j01.x, j1 = j01.y, j2 = j23.x, j3 = j23.y, j4 = j45.x, j5 = j45.y;
+#pragma unroll 1
+    for (int r = 0; r < 6; r += 2) {
+      const double2 cav = load2(o + r), cbv = load2(o + 6 + r);
+      R z[6];
 #pragma unroll
-    for (int r = 0; r < 6; ++r) {
-      const R ca = o[r], cb = o[6 + r];
-      // Y = (Jc^T Jp) w   (ba.rs:249)
-      const R y0 = (ca * j0 + cb * j3) * w;
-      const R y1 = (ca * j1 + cb * j4) * w;
-      const R y2 = (ca * j2 + cb * j5) * w;
-      Z[3 * r + 0] = y0 * l00 + y1 * l10 + y2 * l20;
-      Z[3 * r + 1] = y1 * l11 + y2 * l21;
-      Z[3 * r + 2] = y2 * l22;
-      gs[r] = y0 * t0 + y1 * t1 + y2 * t2;
+      for (int h = 0; h < 2; ++h) {
+        const R ca = h ? cav.y : cav.x, cb = h ? cbv.y : cbv.x;
+        // Y = (Jc^T Jp) w   (ba.rs:249)
+        const R y0 = mul_any(sum2(ca, j0, cb, j3), w);
+        const R y1 = mul_any(sum2(ca, j1, cb, j4), w);
+        const R y2 = mul_any(sum2(ca, j2, cb, j5), w);
+        z[3 * h + 0] = fma(y2, l20, sum2(y0, l00, y1, l10));
+        z[3 * h + 1] = sum2(y1, l11, y2, l21);
+        z[3 * h + 2] = mul_any(y2, l22);
+        gs[r + h] = fma(y2, t2, sum2(y0, t0, y1, t1));
+      }
+#pragma unroll
+      for (int i = 0; i < 6; i += 2) store2(Z + 3 * r + i, z[i], z[i + 1]);
     }
     // w Jg^T (Jp t)
-    const R pt0 = j0 * t0 + j1 * t1 + j2 * t2, pt1 = j3 * t0 + j4 * t1 + j5 * t2;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) gs[6 + a] = (o[18 + a] * pt0 + o[21 + a] * pt1) * w;
+    const R pt0 = fma(j2, t2, sum2(j0, t0, j1, t1)), pt1 = fma(j5, t2, sum2(j3, t0, j4, t1));
+#pragma unroll 1
+    for (int a = 0; a < 3; ++a) gs[6 + a] = mul_any(sum2(o[18 + a], pt0, o[21 + a], pt1), w);
   }
-  // Lens entries: Y_g = sum over the point's observations in group g (ba.rs:251-259).
-  const uint32_t l0 = S.lens_ptr[p], l1 = S.lens_ptr[p + 1];
+  // Lens entries: the first one's sum is done, further ones take a pass each.
   for (uint32_t j = l0; j < l1; ++j) {
-    R Y[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (uint32_t k = s; k < e; ++k) {
+    if (j > l0)
+#pragma unroll
+      for (int i = 0; i < 9; ++i) Y[i] = (R)0;
+    for (uint32_t k = j > l0 ? s : e; k < e; ++k) {
       if (S.obs_lens[k] != j) continue;
       const R* o = B.lin + (size_t)k * kLinW;
       if (o[27] == (R)0) continue;

@@ -23,7 +23,7 @@ namespace ba {
 
 // Exponent field 512 .. 1532: the product's is 1 .. 2042.
 BA_MUL_FN bool mul_safe_hi(uint32_t hi) {
-  return ((hi >> 20) & 0x7ffu) - 512u < 1021u;
+  return hi * 2u - (512u << 21) < (1021u << 21);
 }
 
 // A factor: its significand in the upper 53 of 64 bits, and sign and exponent
@@ -62,6 +62,11 @@ __device__ __forceinline__ MulOp mul_op(double x) {
 }
 __device__ __forceinline__ double mul_int(const MulOp& a, const MulOp& b) {
   return __longlong_as_double((long long)mul_bits(a, b));
+}
+// The rounded product of any two doubles, in integers where they allow it.
+__device__ __forceinline__ double mul_any(double a, double b) {
+  if (mul_safe(a) && mul_safe(b)) return mul_int(mul_op(a), mul_op(b));
+  return __dmul_rn(a, b);
 }
 #endif
 
