@@ -35,6 +35,31 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// Warp sum of N values per lane by halving: after the offsets 16, 8, 4, 2, 1
+// the lane holds the totals of values off .. off + cnt - 1 in out[].
+template <int O, int N, int M, typename R>
+__device__ __forceinline__ void warp_halve(const R (&v)[N], int lane, int& off, int& cnt,
+                                           R (&out)[M]) {
+  if constexpr (O == 0) {
+    static_assert(N <= M, "results per lane");
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = v[i];
+  } else {
+    constexpr int H = (N + 1) / 2;
+    const bool up = lane & O;
+    R w[H];
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      const int j = H + i < N ? H + i : i;  // (odd N: an upper lane's last one is not used)
+      const R recv = __shfl_xor_sync(kFull, up ? v[i] : v[j], O);
+      w[i] = (up ? v[j] : v[i]) + recv;
+    }
+    off += up ? H : 0;
+    cnt = up ? cnt - H : min(cnt, H);
+    warp_halve<O / 2>(w, lane, off, cnt, out);
+  }
+}
+
 // Deterministic block sum of N values per thread (fixed tree: lanes by
 // butterfly, then warps in index order).  Result valid in thread 0.
 // `scratch` holds N * 32 doubles.

@@ -302,81 +302,112 @@ __device__ void jacobi3(double (&A)[3][3], double (&V)[3][3]) {
   }
 }
 
+// Sum of a value that lanes 0 .. 8 of a warp hold (the others 0), in every lane.
+__device__ __forceinline__ double sum9(double v) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  return __shfl_sync(kFull, v, 0);
+}
+
 // Eigenvector of the smallest eigenvalue of the symmetric positive
-// semi-definite N x N matrix M (row-major, overwritten) by inverse iteration
-// on its pivoted Cholesky factor, from the start vector x (overwritten with
-// the unit result).  A pivot below 1e-30 trace(M) is raised to that floor, so
-// an exactly singular M yields a null vector.  Single thread.  The reference
-// takes this eigenvector from nalgebra's symmetric_eigen (geometry.rs:209-215)
-// and the rank-2 step's right singular vector from its SVD (:216-221); any
-// accurate method gives it up to sign and rounding when the smallest
-// eigenvalue is simple.
-template <int N>
-__device__ void smallest_eigvec(double* M, double* x) {
-  int perm[N];
-  double tr = 0.0;
-  for (int i = 0; i < N; ++i) perm[i] = i, tr += M[(N + 1) * i];
+// semi-definite 9 x 9 matrix M (row-major, in shared memory, overwritten) by
+// inverse iteration on its pivoted Cholesky factor.  A pivot below 1e-30
+// trace(M) is raised to that floor, so an exactly singular M yields a null
+// vector.  The reference takes this eigenvector from nalgebra's
+// symmetric_eigen (geometry.rs:209-215); any accurate method gives it up to
+// sign and rounding when the smallest eigenvalue is simple.
+//
+// By a warp: lane i < 9 has row i of the factor's column, of the solves and of
+// the result x_i, which it returns; the 36 entries that a column changes are a
+// lane's each (four of them a second one).  On one thread the same 1200
+// operations and more took half of the pair's time.
+__device__ double smallest_eigvec9(double* M) {
+  const int lane = threadIdx.x & 31;
+  const bool row = lane < 9;
+  const int li = row ? lane : 0;
+  // entries (ei, ej), 1 <= ej <= ei <= 8, number e = ei (ei - 1) / 2 + ej - 1
+  int ei[2], ej[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    int e = lane + 32 * h;
+    ei[h] = 1;
+    while (e >= ei[h] && ei[h] < 9) e -= ei[h], ++ei[h];
+    ej[h] = e + 1;  // (ei 9: none)
+  }
+  const double tr = sum9(row ? M[10 * li] : 0.0);
   const double floor_d = 1e-30 * tr + 1e-300;
-  double rdiag[N];
-  for (int k = 0; k < N; ++k) {
-    int pk = k;
-    for (int i = k + 1; i < N; ++i)
-      if (M[(N + 1) * i] > M[(N + 1) * pk]) pk = i;
-    if (pk != k) {  // symmetric swap of rows/columns k and pk
-      for (int j = 0; j < N; ++j) {
-        const double t = M[N * k + j];
-        M[N * k + j] = M[N * pk + j], M[N * pk + j] = t;
-      }
-      for (int j = 0; j < N; ++j) {
-        const double t = M[N * j + k];
-        M[N * j + k] = M[N * j + pk], M[N * j + pk] = t;
-      }
-      const int t = perm[k];
-      perm[k] = perm[pk], perm[pk] = t;
+  int perm = lane;      // column `lane` of the factor is x's entry perm
+  double rdiag = 0.0;   // of row `lane`
+  for (int k = 0; k < 9; ++k) {
+    // The largest remaining diagonal entry, the first of equals (negative ones,
+    // rounding's, count as zero: a positive double's bits are in its order).
+    const double dk = row && lane >= k ? fmax(M[10 * li], 0.0) : 0.0;
+    unsigned long long key = (unsigned long long)__double_as_longlong(dk);
+    int pk = row && lane >= k ? lane : 31;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      const unsigned long long ok = __shfl_xor_sync(kFull, key, o);
+      const int op = __shfl_xor_sync(kFull, pk, o);
+      if (ok > key || (ok == key && op < pk)) key = ok, pk = op;
     }
-    const double lkk = sqrt(fmax(M[(N + 1) * k], floor_d));
-    const double rk = 1.0 / lkk;
-    M[(N + 1) * k] = lkk, rdiag[k] = rk;
-    for (int i = k + 1; i < N; ++i) M[N * i + k] *= rk;
-    for (int i = k + 1; i < N; ++i)
-      for (int j = k + 1; j <= i; ++j) {
-        M[N * i + j] -= M[N * i + k] * M[N * j + k];
-        M[N * j + i] = M[N * i + j];
+    pk = __shfl_sync(kFull, pk, 0);
+    if (pk != k) {  // symmetric swap of rows and columns k and pk
+      if (row) {
+        const double t = M[9 * k + li];
+        M[9 * k + li] = M[9 * pk + li], M[9 * pk + li] = t;
       }
+      __syncwarp();
+      if (row) {
+        const double t = M[9 * li + k];
+        M[9 * li + k] = M[9 * li + pk], M[9 * li + pk] = t;
+      }
+      const int a = __shfl_sync(kFull, perm, k), b = __shfl_sync(kFull, perm, pk);
+      perm = lane == k ? b : lane == pk ? a : perm;
+      __syncwarp();
+    }
+    const double lkk = sqrt(fmax(M[10 * k], floor_d));
+    const double rk = __drcp_rn(lkk);
+    if (lane == k) rdiag = rk;
+    __syncwarp();
+    if (row && lane > k) M[9 * li + k] *= rk;
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (ei[h] < 9 && ej[h] > k) {
+        const double v = M[9 * ei[h] + ej[h]] - M[9 * ei[h] + k] * M[9 * ej[h] + k];
+        M[9 * ei[h] + ej[h]] = v, M[9 * ej[h] + ei[h]] = v;
+      }
+    __syncwarp();
   }
-  // L in the lower triangle: P^T M P = L L^T.
-  double nx = 0.0;
-  for (int i = 0; i < N; ++i) nx += x[i] * x[i];
-  if (!(nx > 1e-300) || !(nx < 1e300)) {  // zero or non-finite start: a generic one
-    nx = 0.0;
-    for (int i = 0; i < N; ++i) x[i] = 1.0 - 0.0625 * i, nx += x[i] * x[i];
-  }
-  nx = 1.0 / sqrt(nx);
-  for (int i = 0; i < N; ++i) x[i] *= nx;
+  // L in the lower triangle: P^T M P = L L^T.  The iterate in the factor's
+  // order: lane i has entry perm of x.
+  double x = row ? 1.0 - 0.0625 * perm : 0.0;
+  x *= rsqrt(sum9(x * x));
   for (int it = 0; it < 60; ++it) {
-    double y[N];
-    for (int i = 0; i < N; ++i) y[i] = x[perm[i]];
-    for (int i = 0; i < N; ++i) {  // L z = P^T x
-      double a = y[i];
-      for (int j = 0; j < i; ++j) a -= M[N * i + j] * y[j];
-      y[i] = a * rdiag[i];
+    double y = x;
+    for (int j = 0; j < 9; ++j) {  // L z = x
+      const double z = __shfl_sync(kFull, y * rdiag, j);
+      y = lane == j ? z : row && lane > j ? y - M[9 * li + j] * z : y;
     }
-    for (int i = N - 1; i >= 0; --i) {  // L^T w = z
-      double a = y[i];
-      for (int j = i + 1; j < N; ++j) a -= M[N * j + i] * y[j];
-      y[i] = a * rdiag[i];
+    for (int j = 8; j >= 0; --j) {  // L^T w = z
+      const double w = __shfl_sync(kFull, y * rdiag, j);
+      y = lane == j ? w : lane < j ? y - M[9 * j + li] * w : y;
     }
-    double z[N], nn = 0.0;
-    for (int i = 0; i < N; ++i) z[perm[i]] = y[i];
-    for (int i = 0; i < N; ++i) nn += z[i] * z[i];
-    nn = 1.0 / sqrt(nn);
-    double dot = 0.0;
-    for (int i = 0; i < N; ++i) z[i] *= nn, dot += z[i] * x[i];
-    const double sg = dot < 0.0 ? -1.0 : 1.0;
-    double diff = 0.0;
-    for (int i = 0; i < N; ++i) diff = fmax(diff, fabs(sg * z[i] - x[i])), x[i] = sg * z[i];
-    if (diff <= 1e-15) break;
+    y = row ? y : 0.0;
+    y *= rsqrt(sum9(y * y));
+    if (sum9(y * x) < 0.0) y = -y;
+    const bool done = !row || fabs(y - x) <= 1e-15;
+    x = y;
+    if (__all_sync(kFull, done)) break;
   }
+  // back to x's own order
+  double out = 0.0;
+  for (int j = 0; j < 9; ++j) {
+    const double v = __shfl_sync(kFull, x, j);
+    const int at = __shfl_sync(kFull, perm, j);
+    if (lane == at) out = v;
+  }
+  return out;
 }
 
 // Rank 2, denormalisation and unit norm of the 8-point solution f
@@ -853,8 +884,10 @@ __device__ __forceinline__ double cta_sum_d(double v, double* red) {
 // CTA per pair: the best hypothesis (the first with the most inliers), its
 // inliers, and one refit on them (geometry.rs:286-298), kept when it has at
 // least as many inliers.  The refit's centroid, mean distance and normal
-// matrix are CTA reductions in a fixed order; its eigenvector comes from
-// smallest_eigvec9.
+// matrix are CTA reductions in a fixed order (the 45 sums by halving: 48
+// additions a lane for 225); its eigenvector is a warp's work, another one in
+// each CTA so that an SM's CTAs spread it over its four FP64 pipes.  1603
+// pairs of 150 cameras: 1.13 -> 0.89 ms.
 __global__ void __launch_bounds__(kRefitThreads) ransac_select_kernel(RansacArgs A) {
   __shared__ uint64_t red[kRefitThreads / 32 + 1];
   __shared__ int wsum[kRefitThreads / 32];
@@ -919,13 +952,12 @@ __global__ void __launch_bounds__(kRefitThreads) ransac_select_kernel(RansacArgs
       for (int c = r; c < 9; ++c) acc[k++] += row[r] * row[c];
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int off = 0, cnt45 = 45;
+  double v2[2];
+  warp_halve<16>(acc, lane, off, cnt45, v2);
 #pragma unroll
-  for (int k = 0; k < 45; ++k) {
-    double v = acc[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    if (lane == 0) msum[warp][k] = v;
-  }
+  for (int i = 0; i < 2; ++i)
+    if (i < cnt45) msum[warp][off + i] = v2[i];
   __syncthreads();
   if (threadIdx.x < 45) {
     double t = 0.0;
@@ -936,16 +968,18 @@ __global__ void __launch_bounds__(kRefitThreads) ransac_select_kernel(RansacArgs
     Ms[9 * r + c] = t, Ms[9 * c + r] = t;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (warp == (int)(blockIdx.x % (kRefitThreads / 32))) {
+    const double x = smallest_eigvec9(Ms);
     double fm[9], F[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) fm[i] = 1.0 - 0.0625 * i;
-    smallest_eigvec<9>(Ms, fm);
-    const double ta[9] = {sA, 0.0, -sA * max_, 0.0, sA, -sA * may, 0.0, 0.0, 1.0};
-    const double tb[9] = {sB, 0.0, -sB * mbx, 0.0, sB, -sB * mby, 0.0, 0.0, 1.0};
-    ok_s = ep_finish(fm, ta, tb, F);
-    if (ok_s)
-      for (int j = 0; j < 9; ++j) Fs[j] = F[j];
+    for (int i = 0; i < 9; ++i) fm[i] = __shfl_sync(kFull, x, i);
+    if (lane == 0) {
+      const double ta[9] = {sA, 0.0, -sA * max_, 0.0, sA, -sA * may, 0.0, 0.0, 1.0};
+      const double tb[9] = {sB, 0.0, -sB * mbx, 0.0, sB, -sB * mby, 0.0, 0.0, 1.0};
+      ok_s = ep_finish(fm, ta, tb, F);
+      if (ok_s)
+        for (int j = 0; j < 9; ++j) Fs[j] = F[j];
+    }
   }
   __syncthreads();
   if (!ok_s) return;

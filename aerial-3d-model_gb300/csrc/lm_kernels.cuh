@@ -1985,31 +1985,6 @@ struct SchurOut {
   static constexpr int kN = kSym ? kRows * (kRows + 1) / 2 : kRows * kCols;
 };
 
-// Warp sum of N values per lane by halving: after the offsets 16, 8, 4, 2, 1
-// the lane holds the totals of values off .. off + cnt - 1 in out[].
-template <int O, int N, int M, typename R>
-__device__ __forceinline__ void warp_halve(const R (&v)[N], int lane, int& off, int& cnt,
-                                           R (&out)[M]) {
-  if constexpr (O == 0) {
-    static_assert(N <= M, "results per lane");
-#pragma unroll
-    for (int i = 0; i < N; ++i) out[i] = v[i];
-  } else {
-    constexpr int H = (N + 1) / 2;
-    const bool up = lane & O;
-    R w[H];
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-      const int j = H + i < N ? H + i : i;  // (odd N: an upper lane's last one is not used)
-      const R recv = __shfl_xor_sync(kFull, up ? v[i] : v[j], O);
-      w[i] = (up ? v[j] : v[i]) + recv;
-    }
-    off += up ? H : 0;
-    cnt = up ? cnt - H : min(cnt, H);
-    warp_halve<O / 2>(w, lane, off, cnt, out);
-  }
-}
-
 // The sum over pairs [b, e) of a destination block into part[36].
 template <SchurKind K, typename R>
 __device__ __forceinline__ void schur_segment(const Prob& P, const StructView& S,
