@@ -51,10 +51,10 @@ __device__ __forceinline__ void obs_vjp(const Prob& P, const StateView& st, int6
   }
   const double f = K[0], k1 = K[3], k2 = K[4];
   const double iz = __drcp_rn(xc[2]);
-  const double px = xc[0] * iz, py = xc[1] * iz;
-  const double r2 = px * px + py * py;
-  const double d = 1.0 + k1 * r2 + k2 * r2 * r2;
-  const double qx = px * d, qy = py * d;
+  const double px = mul_any(xc[0], iz), py = mul_any(xc[1], iz);
+  const double r2 = sum2(px, px, py, py);
+  const double d = fma(mul_any(k2, r2), r2, fma(k1, r2, 1.0));
+  const double qx = mul_any(px, d), qy = mul_any(py, d);
   // e = u - pred: the prediction's cotangent is the residual's negative
   double l0, l1;
   if (cot) {
@@ -62,25 +62,25 @@ __device__ __forceinline__ void obs_vjp(const Prob& P, const StateView& st, int6
   } else {  // d rho / d e = rho'(|e|^2) * 2 e, rho' = the IRLS weight
     const double ex = P.obs_uv[2 * k] - (f * qx + K[1]);
     const double ey = P.obs_uv[2 * k + 1] - (f * qy + K[2]);
-    const double w = -2.0 * robust_weight(ex * ex + ey * ey, sigma, P.loss);
-    l0 = w * ex, l1 = w * ey;
+    const double w = -2.0 * robust_weight(sum2(ex, ex, ey, ey), sigma, P.loss);
+    l0 = mul_any(w, ex), l1 = mul_any(w, ey);
   }
-  const double s = l0 * px + l1 * py;
-  o.in[0] = l0 * qx + l1 * qy;
+  const double s = sum2(l0, px, l1, py);
+  o.in[0] = sum2(l0, qx, l1, qy);
   o.in[1] = l0;
   o.in[2] = l1;
-  o.in[3] = f * r2 * s;
-  o.in[4] = o.in[3] * r2;
+  o.in[3] = mul_any(mul_any(f, r2), s);
+  o.in[4] = mul_any(o.in[3], r2);
   if constexpr (kGeo) {
-    const double cs = 2.0 * (k1 + 2.0 * k2 * r2) * s;
-    const double fz = f * iz;
-    const double g0 = (d * l0 + cs * px) * fz, g1 = (d * l1 + cs * py) * fz;
-    const double g2 = -(g0 * px + g1 * py);
-    o.rot[0] = xc[1] * g2 - xc[2] * g1;
-    o.rot[1] = xc[2] * g0 - xc[0] * g2;
-    o.rot[2] = xc[0] * g1 - xc[1] * g0;
+    const double cs = mul_any(fma(4.0 * k2, r2, k1 + k1), s);
+    const double fz = mul_any(f, iz);
+    const double g0 = mul_any(sum2(d, l0, cs, px), fz), g1 = mul_any(sum2(d, l1, cs, py), fz);
+    const double g2 = -sum2(g0, px, g1, py);
+    o.rot[0] = fma(xc[1], g2, -mul_any(xc[2], g1));
+    o.rot[1] = fma(xc[2], g0, -mul_any(xc[0], g2));
+    o.rot[2] = fma(xc[0], g1, -mul_any(xc[1], g0));
 #pragma unroll
-    for (int j = 0; j < 3; ++j) o.pt[j] = R[j] * g0 + R[3 + j] * g1 + R[6 + j] * g2;
+    for (int j = 0; j < 3; ++j) o.pt[j] = fma(R[6 + j], g2, sum2(R[j], g0, R[3 + j], g1));
   }
 }
 

@@ -76,14 +76,14 @@ __device__ __forceinline__ void mul3(const double* A, const double* B, double* C
 // sampson (geometry.rs:233-246).
 __device__ __forceinline__ double ep_sampson(const double* F, double ax, double ay, double bx,
                                              double by) {
-  const double f0 = F[0] * ax + F[1] * ay + F[2];
-  const double f1 = F[3] * ax + F[4] * ay + F[5];
-  const double f2 = F[6] * ax + F[7] * ay + F[8];
-  const double g0 = F[0] * bx + F[3] * by + F[6];
-  const double g1 = F[1] * bx + F[4] * by + F[7];
-  const double e = bx * f0 + by * f1 + f2;
-  const double d = f0 * f0 + f1 * f1 + g0 * g0 + g1 * g1;
-  return d < 1e-18 ? kF64Max : e * e / d;
+  const double f0 = fma(F[0], ax, fma(F[1], ay, F[2]));
+  const double f1 = fma(F[3], ax, fma(F[4], ay, F[5]));
+  const double f2 = fma(F[6], ax, fma(F[7], ay, F[8]));
+  const double g0 = fma(F[0], bx, fma(F[3], by, F[6]));
+  const double g1 = fma(F[1], bx, fma(F[4], by, F[7]));
+  const double e = fma(bx, f0, fma(by, f1, f2));
+  const double d = fma(g1, g1, fma(g0, g0, sum2(f0, f0, f1, f1)));
+  return d < 1e-18 ? kF64Max : mul_any(e, e) / d;
 }
 
 // ---- RANSAC -------------------------------------------------------------------

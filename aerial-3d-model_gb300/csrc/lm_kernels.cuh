@@ -115,11 +115,6 @@ __device__ __forceinline__ double robust_rho(double e2, double sigma, int loss) 
 // compare so (an integer compare instead of an FP64 one).
 constexpr long long kQMaxBits = 0x7e37e43c8800759cLL;
 
-// a b + c d as the compiler fuses it: the second product is rounded.
-__device__ __forceinline__ double sum2(double a, double b, double c, double d) {
-  return fma(a, b, mul_any(c, d));
-}
-
 // linearise (ba.rs:56-101) of observation k into out[kLinW]; false if the
 // point is not in front of the camera (z <= 1e-6).
 template <typename R>

@@ -68,6 +68,10 @@ __device__ __forceinline__ double mul_any(double a, double b) {
   if (mul_safe(a) && mul_safe(b)) return mul_int(mul_op(a), mul_op(b));
   return __dmul_rn(a, b);
 }
+// a b + c d as the compiler fuses it: the second product is rounded.
+__device__ __forceinline__ double sum2(double a, double b, double c, double d) {
+  return fma(a, b, mul_any(c, d));
+}
 #endif
 
 }  // namespace ba

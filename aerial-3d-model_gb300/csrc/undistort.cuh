@@ -4,11 +4,14 @@
 // The steps are FP64 operations one after the other, ~64 cycles of the SM
 // sub-partition each, and a division is nine of them; the two of a step share
 // their divisor.  So a step takes one reciprocal (five) and two residual
-// corrections (three each): 16 operations instead of 23 with the polynomial.
+// corrections (three each): 16 operations instead of 23 with the polynomial,
+// of which the four plain products are made in integers.
 #pragma once
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include "mul_int.cuh"
 
 namespace ba {
 
@@ -20,7 +23,7 @@ static __device__ __noinline__ double quotient_slow(double x, double d) { return
 // residual is exact where neither it nor q leaves the normal range; outside
 // of 2^-900 .. 2^900 (and for zero, infinite or NaN values) the division.
 __device__ __forceinline__ double quotient_by(double x, double d, double r) {
-  const double q = x * r;
+  const double q = mul_any(x, r);
   const uint32_t eq = ((uint32_t)__double2hiint(q) >> 20) & 0x7ffu;
   const uint32_t er = ((uint32_t)__double2hiint(r) >> 20) & 0x7ffu;
   if (eq - 123u > 1800u || er - 123u > 1800u) return quotient_slow(x, d);
@@ -35,8 +38,8 @@ __device__ __forceinline__ void undistort(const double* K, double rf, double u, 
   double px = qx, py = qy;
 #pragma unroll 1
   for (int i = 0; i < 8; ++i) {
-    const double r2 = px * px + py * py;
-    const double d = 1.0 + k1 * r2 + k2 * r2 * r2;
+    const double r2 = sum2(px, px, py, py);
+    const double d = fma(mul_any(k2, r2), r2, fma(k1, r2, 1.0));
     const double r = __drcp_rn(d);
     px = quotient_by(qx, d, r);
     py = quotient_by(qy, d, r);
