@@ -73,17 +73,28 @@ __device__ __forceinline__ void mul3(const double* A, const double* B, double* C
       C[3 * i + j] = A[3 * i] * B[j] + A[3 * i + 1] * B[3 + j] + A[3 * i + 2] * B[6 + j];
 }
 
-// sampson (geometry.rs:233-246).
+// a x + b y + c.  Fused throughout, or with the rounding of the products of
+// the plain expression, two of the FP64 pipe's operations either way.
+template <bool kFused>
+__device__ __forceinline__ double affine(double a, double x, double b, double y, double c) {
+  return kFused ? fma(a, x, fma(b, y, c)) : sum2(a, x, b, y) + c;
+}
+
+// sampson (geometry.rs:233-246).  The inlier tests take the fused form, for
+// its shorter code in their kernels (the count 2.15 ms, with the other 2.46);
+// the pair check, whose errors are results, keeps the plain expression's
+// roundings.
+template <bool kFused>
 __device__ __forceinline__ double ep_sampson(const double* F, double ax, double ay, double bx,
                                              double by) {
-  const double f0 = fma(F[0], ax, fma(F[1], ay, F[2]));
-  const double f1 = fma(F[3], ax, fma(F[4], ay, F[5]));
-  const double f2 = fma(F[6], ax, fma(F[7], ay, F[8]));
-  const double g0 = fma(F[0], bx, fma(F[3], by, F[6]));
-  const double g1 = fma(F[1], bx, fma(F[4], by, F[7]));
-  const double e = fma(bx, f0, fma(by, f1, f2));
+  const double f0 = affine<kFused>(F[0], ax, F[1], ay, F[2]);
+  const double f1 = affine<kFused>(F[3], ax, F[4], ay, F[5]);
+  const double f2 = affine<kFused>(F[6], ax, F[7], ay, F[8]);
+  const double g0 = affine<kFused>(F[0], bx, F[3], by, F[6]);
+  const double g1 = affine<kFused>(F[1], bx, F[4], by, F[7]);
+  const double e = affine<kFused>(bx, f0, by, f1, f2);
   const double d = fma(g1, g1, fma(g0, g0, sum2(f0, f0, f1, f1)));
-  return d < 1e-18 ? kF64Max : mul_any(e, e) / d;
+  return d < 1e-18 ? kF64Max : quotient_by(mul_any(e, e), d, reciprocal_near(d));
 }
 
 // ---- RANSAC -------------------------------------------------------------------
@@ -777,7 +788,7 @@ __global__ void __launch_bounds__(kCountThreads) ransac_count_kernel(RansacArgs 
               int r = inlier_fp32(H, tile[i], t2);
               if (r < 0) {
                 const double* u64 = A.uv + 4 * ((size_t)b + t0 + i);
-                r = ep_sampson(A.F + 9 * h, u64[0], u64[1], u64[2], u64[3]) < A.t2;
+                r = ep_sampson<true>(A.F + 9 * h, u64[0], u64[1], u64[2], u64[3]) < A.t2;
               }
               in[j] = r != 0;
             }
@@ -851,7 +862,7 @@ __device__ int mark_inliers(const double* F, const double* uv, uint32_t n, doubl
     bool in = false;
     if (i < n) {
       const double* u = uv + 4 * (size_t)i;
-      in = ep_sampson(F, u[0], u[1], u[2], u[3]) < t2;
+      in = ep_sampson<true>(F, u[0], u[1], u[2], u[3]) < t2;
       flag[i] = in;
     }
     const unsigned m = __ballot_sync(kFull, in);
@@ -986,7 +997,7 @@ __global__ void __launch_bounds__(kRefitThreads) ransac_select_kernel(RansacArgs
   int cnt = 0;
   for (uint32_t i = threadIdx.x; i < n; i += kRefitThreads) {
     const double* u = U + 4 * (size_t)i;
-    list[i] = ep_sampson(Fs, u[0], u[1], u[2], u[3]) < A.t2;  // (the index list is done with)
+    list[i] = ep_sampson<true>(Fs, u[0], u[1], u[2], u[3]) < A.t2;  // (the index list is done with)
     cnt += list[i];
   }
   const int nr = cta_sum_int(cnt, wsum);
@@ -1017,7 +1028,8 @@ constexpr uint32_t kFitKeys = 3072;  // total-order keys of a pair in shared mem
 // then every match's error sqrt(sampson) * f_a on undistorted coordinates,
 // and the pair's median error (element n/2 in total order).
 //
-// Bound by its FP64 operations (~320 a match).  The median is selected in the
+// Bound by its FP64 operations (~190 a match, and as many again in integer
+// instructions: 3.46 -> 2.19 ms for 4.6 million matches).  The median is selected in the
 // CTA that made the errors: sorting all matches by error and then by pair took
 // nine passes over memory (1.3 of 5.6 ms for 4.6 million matches), and the
 // errors 4.1 ms with two divisions a step of the undistortion.
@@ -1065,7 +1077,7 @@ __global__ void __launch_bounds__(kFitsThreads) pair_fits_kernel(FitsArgs A) {
     double x1[2], x2[2];
     undistort(Ka, rfa, ua.x, ua.y, x1);
     undistort(Kb, rfb, ub.x, ub.y, x2);
-    const double err = sqrt(ep_sampson(E, x1[0], x1[1], x2[0], x2[1])) * Ka[0];
+    const double err = sqrt(ep_sampson<false>(E, x1[0], x1[1], x2[0], x2[1])) * Ka[0];
     key[i] = total_order_key(err);
   }
   __syncthreads();
