@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(32) ransac_sample_kernel(RansacArgs A,
 // 4 a^2)) with a = A_pq, d = A_qq - A_pp and the sign of a d, moves t a
 // between the two diagonal entries (Golub and Van Loan, Matrix Computations,
 // 8.5): some 46 FP64 operations where rotating rows and columns and dividing
-// by 2 a took 81 (the fit of 150 pairs by 1000 samples: 3.24 -> 2.62 ms).  An
+// by 2 a took 81 (the fit of 1603 pairs by 600 samples: 3.24 -> 2.62 ms).  An
 // off-diagonal entry below 1e-140 is left (A has a trace near 1 here, and
 // the loop ends when they are below 1e-17).
 __device__ void jacobi3(double (&A)[3][3], double (&V)[3][3]) {
@@ -705,7 +705,7 @@ __device__ __forceinline__ void inlier_tile(const Hyp32& H, const TileBound& B, 
 // tests).  gridDim.x / pairs CTAs share a pair, a bound each.  Four tests a
 // lane are in flight, and both outcomes of a test are formed without a
 // branch.  1603 pairs x 600 x 1300 tests: 3.9 ms with every test made, four
-// hypotheses a warp.
+// hypotheses a warp; now 2.15 ms.
 __global__ void __launch_bounds__(kCountThreads) ransac_count_kernel(RansacArgs A,
                                                                      const float4* uv32,
                                                                      int parts) {
@@ -1029,8 +1029,8 @@ constexpr uint32_t kFitKeys = 3072;  // total-order keys of a pair in shared mem
 // and the pair's median error (element n/2 in total order).
 //
 // Bound by its FP64 operations (~190 a match, and as many again in integer
-// instructions: 3.46 -> 2.19 ms for 4.6 million matches).  The median is selected in the
-// CTA that made the errors: sorting all matches by error and then by pair took
+// instructions: 3.46 -> 2.19 ms for 4.6 million matches).  The median is
+// selected in the CTA that made the errors: sorting all matches by error and then by pair took
 // nine passes over memory (1.3 of 5.6 ms for 4.6 million matches), and the
 // errors 4.1 ms with two divisions a step of the undistortion.
 __global__ void __launch_bounds__(kFitsThreads) pair_fits_kernel(FitsArgs A) {
@@ -1220,8 +1220,8 @@ extern "C" ba_status ba_ransac_fundamental(const ba_pair_matches* m, double thre
     DevBuf<uint8_t> valid(ch, s);
     DevBuf<int32_t> count(ch, s);
     DevBuf<float4> uv32(std::max<int64_t>(nm, 1), s);
-    // Counting: two CTAs a pair (1603 pairs of unequal size: 2.25 ms; one 2.45,
-    // three 2.28), more where that leaves SMs with fewer than four, but at
+    // Counting: two CTAs a pair (1603 pairs of unequal size: 2.15 ms; one took
+    // 0.2 ms more, three 0.03), more where that leaves SMs with fewer than four, but at
     // least eight hypotheses a warp, so that the bound of a CTA's first counts
     // serves most of its hypotheses.
     int dev = 0, n_sm = 0;
@@ -1274,9 +1274,9 @@ extern "C" ba_status ba_pair_fits(const ba_pair_matches* m, const double* rot, c
     DevBuf<double> med(std::max<int64_t>(np, 1), s);
     // The correspondences of a large call come in on a second stream, a
     // quarter first: the rest is copied while its pairs are worked on (the copy
-    // is 1.0 ms for 4.6 million, the arithmetic 3.0).  More pieces cost more in
-    // half-empty last waves than they hide (4.35 ms in three, 5.1 in five, 8.9
-    // in seventeen, against 4.3 in one).
+    // is 1.0 ms for 4.6 million, the arithmetic 2.2).  More pieces cost more in
+    // half-empty last waves than they hide (with arithmetic of 3.0 ms: 4.35 ms in
+    // three, 5.1 in five, 8.9 in seventeen, against 4.3 in one).
     std::vector<uint32_t> ptr((size_t)np + 1, 0);
     check(cudaMemcpyAsync(ptr.data(), P.match_ptr.p, 4 * ptr.size(), cudaMemcpyDeviceToHost, s), "d2h");
     check(cudaStreamSynchronize(s), "pair offsets");

@@ -1355,8 +1355,8 @@ constexpr int kCamN = 45;  // 21 U | 18 X | 6 lens U
 // the camera ordering.  Bound by the FP64 operations, 64 cycles of an SM
 // sub-partition each: a CTA per camera left most SMs idle below 152 cameras
 // and filled them unevenly above (500 cameras: 4 on some, 3 on others, at 188
-// registers).  500 cameras with 2.6 M observations: 1142 -> 866 us (1022 with all operations on the FP64 pipe); 77 with
-// 0.26 M: 268 -> 122.
+// registers).  500 cameras with 2.6 M observations: 1142 -> 866 us (1022 with
+// all operations on the FP64 pipe); 77 with 0.26 M: 268 -> 122.
 constexpr int kCamUnits = 8;
 struct CamPair {
   int p, q;

@@ -16,8 +16,9 @@
 // exchange is then one store and one load through L2 with no fence, no
 // arrival counter and no second round trip for the values behind it, and the
 // neighbours' z are gathered while the reductions are still on their way.
-// Measured on the 500-camera survey (FP64, 126 CTAs): 13.4 µs per iteration
-// with a counter barrier and separate partials; on 13 block rows 11.1 µs.
+// Measured (FP64, per iteration; with a counter barrier and separate partials
+// -> now): 500 cameras, 126 CTAs, 13.5 -> 11.5 µs; 77 cameras, 20 CTAs,
+// 11.7 -> 9.0 µs; 12 cameras, 4 CTAs, 9.9 -> 7.4 µs.
 //
 // A CTA keeps its rows' state (x, r, z, p, q and the 6x6 block-Jacobi
 // inverse) in shared memory for the whole solve, and its S blocks too when
