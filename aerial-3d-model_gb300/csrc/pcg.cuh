@@ -18,7 +18,7 @@
 // neighbours' z are gathered while the reductions are still on their way.
 // Measured (FP64, per iteration; with a counter barrier and separate partials
 // -> now): 500 cameras, 126 CTAs, 13.5 -> 11.5 µs; 77 cameras, 20 CTAs,
-// 11.7 -> 9.0 µs; 12 cameras, 4 CTAs, 9.9 -> 7.4 µs.
+// 11.7 -> 9.0 µs; 12 cameras, 4 CTAs, 9.9 -> 7.0 µs (and 6.0 in halves, below).
 //
 // A CTA keeps its rows' state (x, r, z, p, q and the 6x6 block-Jacobi
 // inverse) in shared memory for the whole solve, and its S blocks too when
@@ -515,16 +515,11 @@ __device__ __forceinline__ bool pcg_exchange(const PcgArgs<R>& A, const PcgJob& 
 // 8, 4, 2, 1): afterwards lane sum6_lane(k) holds the sum of value k.  Eight
 // adds; six -> three -> two (one) -> one value per lane.
 __host__ __device__ constexpr int sum6_lane(int k) { return k < 3 ? 4 * k : 4 * k + 4; }
+// From the second step: lanes 0 .. 15 hold values 0, 1, 2 in a, the others 3, 4, 5.
 template <typename T>
-__device__ __forceinline__ T warp_sum6(const T (&v)[6]) {
+__device__ __forceinline__ T warp_sum3(const T (&a)[3]) {
   const int lane = threadIdx.x & 31;
-  const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
-  T a[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const T recv = __shfl_xor_sync(kFull, u16 ? v[i] : v[3 + i], 16);
-    a[i] = (u16 ? v[3 + i] : v[i]) + recv;
-  }
+  const bool u8 = lane & 8, u4 = lane & 4;
   // lower: values 0, 1 of the three; upper: value 2
   const T r0 = __shfl_xor_sync(kFull, u8 ? a[0] : a[2], 8);
   const T r1 = __shfl_xor_sync(kFull, a[1], 8);
@@ -534,6 +529,17 @@ __device__ __forceinline__ T warp_sum6(const T (&v)[6]) {
   c += __shfl_xor_sync(kFull, c, 2);
   c += __shfl_xor_sync(kFull, c, 1);
   return c;
+}
+template <typename T>
+__device__ __forceinline__ T warp_sum6(const T (&v)[6]) {
+  const bool u16 = threadIdx.x & 16;
+  T a[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const T recv = __shfl_xor_sync(kFull, u16 ? v[i] : v[3 + i], 16);
+    a[i] = (u16 ? v[3 + i] : v[i]) + recv;
+  }
+  return warp_sum3(a);
 }
 
 // Blocks that a CTA's rows multiply: all of theirs, but only the diagonal one
@@ -553,7 +559,14 @@ __host__ __device__ inline uint32_t pcg_blocks(const uint32_t* row_ptr, const Pc
 // The FP64 form keeps its longest loop rolled (its overhead hides behind the
 // FP64 operations) and shares the exchange and the division as functions:
 // 3.6 µs of a 9.6 µs iteration went into two inlined exchanges before.
-template <typename R, bool kAll>
+//
+// kHalves (FP64, kAll; every row has up to 16 blocks): a block is in lanes l
+// and l + 16, which take three of its rows each: half the operations of the
+// product and one step less of the sum, whose first step would have added the
+// zeros of lanes without a block.  12 cameras: 7.0 -> 6.0 µs an iteration.  A
+// kernel of its own: in one with the other forms it cost those registers and
+// instruction fetches (77 cameras: 9.0 -> 9.7 µs).
+template <typename R, bool kAll, bool kHalves>
 __device__ bool pcg_job(const PcgArgs<R>& A, const PcgJob& J, double* wsm, double* tot,
                         PcgScalars<R>& sc, int* ok_s, R* rs) {
   constexpr bool kWide = sizeof(R) == 8;
@@ -648,10 +661,12 @@ __device__ bool pcg_job(const PcgArgs<R>& A, const PcgJob& J, double* wsm, doubl
   // before the product are on their way.
   R za[6];
   bool ahead = false;
+  const int bl = kHalves ? lane & 15 : lane;  // the lane's block of a row's first
   auto gather_ahead = [&](unsigned long long tag) {
     if (warp >= (int)nrows) return;
-    const uint32_t k = (uint32_t)sM[3 * warp] + lane;
-    if (k < (uint32_t)sM[3 * warp + 1]) z_of(col_of(k), tag, za);
+    const uint32_t b0 = (uint32_t)sM[3 * warp], b1 = (uint32_t)sM[3 * warp + 1];
+    const uint32_t k = b0 + bl;
+    if (k < b1) z_of(col_of(k), tag, za);
     ahead = true;
   };
 
@@ -707,38 +722,72 @@ __device__ bool pcg_job(const PcgArgs<R>& A, const PcgJob& J, double* wsm, doubl
     for (uint32_t lr = warp; lr < nrows; lr += kPcgWarps) {
       R* st = ROW(lr);
       const uint32_t b0 = (uint32_t)sM[3 * lr], b1 = (uint32_t)sM[3 * lr + 1];
-      R acc[6] = {0, 0, 0, 0, 0, 0};
-      for (uint32_t k = b0 + lane; k < b1; k += 32) {
-        R pp[6];
-        if (ahead && lr == (uint32_t)warp && k == b0 + lane) {
+      R q6;
+      if constexpr (kHalves) {
+        const uint32_t k = b0 + bl;
+        R a3[3] = {0, 0, 0}, pp[6];
+        if (k < b1) {
+          if (ahead && lr == (uint32_t)warp) {
 #pragma unroll
-          for (int j = 0; j < 6; ++j) pp[j] = za[j];
-        } else {
-          z_of(col_of(k), tag, pp);
-        }
-        R* pv = p_at(k);
+            for (int j = 0; j < 6; ++j) pp[j] = za[j];
+          } else {
+            z_of(col_of(k), tag, pp);
+          }
+          const R* pv = p_at(k);
 #pragma unroll
-        for (int j = 0; j < 6; ++j) {
-          pp[j] = p_of<R>(pp[j], pv[j], beta);
-          pv[j] = pp[j];
+          for (int j = 0; j < 6; ++j) pp[j] = p_of<R>(pp[j], pv[j], beta);
+          const R* sb = s_at(k) + (lane >= 16 ? 18 : 0);
+#pragma unroll 1
+          for (int i = 0; i < 3; ++i) {
+            R m[6];
+            load_row6(sb + 6 * i, m);
+            R s = (R)0;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) s += m[j] * pp[j];
+            a3[0] = a3[1], a3[1] = a3[2], a3[2] = s;
+          }
         }
-        const R* sb = s_at(k);
-        // acc[i] of the rolled form is always the front of a queue
-        constexpr int kUnroll = kWide ? 1 : 6;
+        __syncwarp();
+        if (lane < 16 && k < b1) {  // both of its lanes have read the block's p
+          R* pv = p_at(k);
+#pragma unroll
+          for (int j = 0; j < 6; ++j) pv[j] = pp[j];
+        }
+        q6 = warp_sum3(a3);
+      } else {
+        R acc[6] = {0, 0, 0, 0, 0, 0};
+        for (uint32_t k = b0 + lane; k < b1; k += 32) {
+          R pp[6];
+          if (ahead && lr == (uint32_t)warp && k == b0 + lane) {
+#pragma unroll
+            for (int j = 0; j < 6; ++j) pp[j] = za[j];
+          } else {
+            z_of(col_of(k), tag, pp);
+          }
+          R* pv = p_at(k);
+#pragma unroll
+          for (int j = 0; j < 6; ++j) {
+            pp[j] = p_of<R>(pp[j], pv[j], beta);
+            pv[j] = pp[j];
+          }
+          const R* sb = s_at(k);
+          // acc[i] of the rolled form is always the front of a queue
+          constexpr int kUnroll = kWide ? 1 : 6;
 #pragma unroll(kUnroll)
-        for (int i = 0; i < 6; ++i) {
-          R m[6];
-          load_row6(sb + 6 * i, m);
-          R s = acc[0];
+          for (int i = 0; i < 6; ++i) {
+            R m[6];
+            load_row6(sb + 6 * i, m);
+            R s = acc[0];
 #pragma unroll
-          for (int j = 0; j < 6; ++j) s += m[j] * pp[j];
+            for (int j = 0; j < 6; ++j) s += m[j] * pp[j];
 #pragma unroll
-          for (int j = 0; j < 5; ++j) acc[j] = acc[j + 1];
-          acc[5] = s;
+            for (int j = 0; j < 5; ++j) acc[j] = acc[j + 1];
+            acc[5] = s;
+          }
         }
+        __syncwarp();
+        q6 = warp_sum6(acc);
       }
-      __syncwarp();
-      const R q6 = warp_sum6(acc);
       // own p = z + β p(prev); S_cg^T p_c of the row's lens block
       const int32_t lp = sM[3 * lr + 2];
       if constexpr (kWide) {
@@ -889,7 +938,7 @@ __device__ bool pcg_job(const PcgArgs<R>& A, const PcgJob& J, double* wsm, doubl
   return true;
 }
 
-template <typename R>
+template <typename R, bool kHalves = false>
 __global__ void __launch_bounds__(kPcgThreads, 2) pcg_kernel(PcgArgs<R> A) {
   __shared__ double wsm[kPcgWarps * 4];
   __shared__ double tot[4];
@@ -908,9 +957,13 @@ __global__ void __launch_bounds__(kPcgThreads, 2) pcg_kernel(PcgArgs<R> A) {
       return;
     }
     const bool all = pcg_blocks(A.row_ptr, J, A.lens_row[J.model]) <= A.smem_blocks;
-    if (all ? !pcg_job<R, true>(A, J, wsm, tot, sc, &ok_s, rs)
-            : !pcg_job<R, false>(A, J, wsm, tot, sc, &ok_s, rs))
-      return;
+    bool on;
+    if constexpr (kHalves)
+      on = pcg_job<R, true, true>(A, J, wsm, tot, sc, &ok_s, rs);
+    else
+      on = all ? pcg_job<R, true, false>(A, J, wsm, tot, sc, &ok_s, rs)
+               : pcg_job<R, false, false>(A, J, wsm, tot, sc, &ok_s, rs);
+    if (!on) return;
   }
 }
 

@@ -524,6 +524,7 @@ struct LmEngine {
   int32_t imp_ncta = 0;
   // Cluster-resident PCG (mixed form).
   bool use_cluster = false;
+  void* pcg_fn = nullptr;  // the grid kernel of the plan
   bool cl_two = false;  // two of the cluster kernel's CTAs per SM
   int cl_size = 0;
   int cl_threads = kCgThreads;  // threads per CTA of the cluster kernel
@@ -956,6 +957,25 @@ struct LmEngine {
     for (const PcgJob& j : plan.jobs)
       most = std::max(most, pcg_blocks(SB.h_row_ptr.data(), j, h_lens[j.model]));
     pblk.alloc(most > smem_blocks ? (size_t)SB.nz * 6 : 1, s);
+    // The form for short rows: all blocks in shared memory, and 16 a row or
+    // fewer (the lens row multiplies one).
+    pcg_fn = (void*)pcg_kernel<R>;
+    if constexpr (sizeof(R) == 8) {
+      bool halves = most <= smem_blocks;
+      for (const PcgJob& j : plan.jobs)
+        for (uint32_t r = j.row0; r < j.row1 && halves; ++r)
+          halves = (int32_t)r == h_lens[j.model] || SB.h_row_ptr[r + 1] - SB.h_row_ptr[r] <= 16;
+      if (halves) {
+        auto* fn = pcg_kernel<R, true>;
+        check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kPcgSmemBudget),
+              "pcg smem");
+        int occ = 0;
+        check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kPcgThreads, kPcgSmemBudget),
+              "occupancy");
+        if ((int64_t)occ * ctx.n_sm >= plan.ncta) pcg_fn = (void*)fn;
+      }
+    }
     check(cudaStreamSynchronize(s), "sync");  // host plan vectors
     pa = PcgArgs<R>{jobs, cta_job0, pcg_epoch, pcg_words, pcg_said, pcg_zx, plan.ncta, SB.row_ptr,
                     SB.col_idx, S, pre, g, x, pblk, lens_row, lens_pos, SB.diag_pos, smem_rows,
@@ -1456,7 +1476,7 @@ struct LmEngine {
             "pcg cluster launch");
     } else {
       void* args[] = {&pa};
-      check(cudaLaunchCooperativeKernel((void*)pcg_kernel<R>, dim3(plan.ncta), dim3(kPcgThreads),
+      check(cudaLaunchCooperativeKernel(pcg_fn, dim3(plan.ncta), dim3(kPcgThreads),
                                         args, smem_bytes, s),
             "pcg launch");
     }

@@ -42,6 +42,8 @@ def network(n_cams, span, n_points, groups, seed):
 @pytest.mark.parametrize("n_cams,span,n_points,groups", [
     (2, 2, 40, 1),        # one CTA
     (12, 5, 300, 1),
+    (40, 8, 500, 1),      # rows of 16 blocks with the lens block
+    (40, 9, 500, 1),      # of 18
     (127, 6, 3000, 1),    # 32 CTAs of four rows: all decide
     (128, 6, 3000, 1),    # 33: the last one decides
     (150, 17, 2500, 1),   # rows of 33 blocks and the lens block
