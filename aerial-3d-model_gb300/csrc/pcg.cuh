@@ -70,8 +70,8 @@ constexpr int kSaidPitch = 8;
 
 // Groups of up to this many CTAs: every CTA collects every partial and forms
 // the totals itself (one hop).  Larger groups: the last CTA (it owns the lens
-// row) collects them, and the others wait for its result (two hops, but no
-// polling of everything by everyone).  Measured with 2 / 4 values per
+// row: the plan gives every CTA of a group rows) collects them, and the others
+// wait for its result (two hops, but no polling of everything by everyone).  Measured with 2 / 4 values per
 // exchange, cycles: 4 CTAs 970 / 1260 against 1920 / 1960; 126 CTAs 2100 /
 // 3620 against 2740 / 2950, and CTAs that arrive early no longer slow the
 // loads of those that are late (126 CTAs inside the solver: 7500 cycles from

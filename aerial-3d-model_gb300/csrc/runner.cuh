@@ -97,6 +97,7 @@ inline PcgPlan plan_pcg(const Context& ctx, const std::vector<uint32_t>& row_ptr
     for (uint32_t r = r0; r < r1; ++r) total += rc[r];
     uint32_t row = r0;
     int64_t acc = 0;
+    int32_t used = 0;
     for (int64_t k = 0; k < g; ++k) {
       const uint32_t start = row;
       const int64_t target = (total * (k + 1)) / g;
@@ -110,11 +111,17 @@ inline PcgPlan plan_pcg(const Context& ctx, const std::vector<uint32_t>& row_ptr
         acc += rc[row];
         ++row;
       }
+      // Rows of many blocks near the end can leave nothing for the last CTAs:
+      // the group ends with the last row (the lens row, whose CTA leads a
+      // large group: pcg_exchange).
+      if (start == row && k > 0) break;
       pl.cta_job0.push_back((int32_t)pl.jobs.size());
-      pl.jobs.push_back(PcgJob{(int32_t)m, (int32_t)k, (int32_t)g, cta, start, row});
+      pl.jobs.push_back(PcgJob{(int32_t)m, (int32_t)k, 0, cta, start, row});
+      ++used;
     }
     if (row != r1) throw std::runtime_error("PCG plan left rows unassigned");
-    cta += (int32_t)g;
+    for (int32_t k = 1; k <= used; ++k) pl.jobs[pl.jobs.size() - k].gsize = used;
+    cta += used;
   }
   pl.ncta = cta;
   pl.cta_job0.push_back((int32_t)pl.jobs.size());
