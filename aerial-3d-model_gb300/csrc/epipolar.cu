@@ -796,9 +796,14 @@ __global__ void __launch_bounds__(kCountThreads) ransac_count_kernel(RansacArgs 
           }
           cnt += __popc(__ballot_sync(kFull, in[j]));
         }
-        // strictly less: of equal counts the first hypothesis wins
+        // Strictly less: of equal counts the first hypothesis wins.  Other
+        // warps raise the bound meanwhile, so one lane reads it for all: lanes
+        // with different values would part before the next ballot.
         const int64_t left = (int64_t)n - t0 - i0 - 32 * kTests;
-        if (left > 0 && cnt + left < *(volatile int*)&best) {
+        int bound = 0;
+        if (lane == 0) bound = *(volatile int*)&best;
+        bound = __shfl_sync(kFull, bound, 0);
+        if (left > 0 && cnt + left < bound) {
           live = false;
           cnt = 0;
           break;
