@@ -182,6 +182,10 @@ __global__ void __launch_bounds__(32) ransac_sample_kernel(RansacArgs A,
       const int left = have - pos;
       if (left > kDraws) {  // a sample that 2048 draws do not fill: not with n >= 12
         if (lane == 0) atomicOr(A.err, ERR_STRUCTURE);
+        for (; it + lane < A.iters; it += 32) {  // (the fit reads every sample)
+          out[2 * (it + lane)] = make_uint4(0, 1, 2, 3);
+          out[2 * (it + lane) + 1] = make_uint4(4, 5, 6, 7);
+        }
         return;
       }
       for (int i0 = 0; i0 < left; i0 += 32) {  // to the front (pos >= 32, or the buffer is empty)
