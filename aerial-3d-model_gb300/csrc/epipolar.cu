@@ -1270,6 +1270,7 @@ extern "C" ba_status ba_pair_fits(const ba_pair_matches* m, const double* rot, c
                                   int64_t n_groups, void* stream, double* median_px) {
   return guarded([&] {
     if (n_cams < 0 || n_groups < 0) throw BadInput("negative size");
+    if (m && m->n_pairs > 0x7fffffff) throw BadInput("too many pairs");  // a CTA each
     if ((n_cams > 0 && (!rot || !center || !cam_group)) || (n_groups > 0 && !intr))
       throw BadInput("null camera array");
     cudaStream_t s = (cudaStream_t)stream;
