@@ -241,10 +241,9 @@ __global__ void __launch_bounds__(kTriThreads) tri_point_kernel(TriArgs T) {
   T.kept[t] = 2;  // triangulated; decided in tri_keep_kernel
 }
 
-// The tracks that tri_point_kernel left, by Jacobi rotations.
-__device__ void tri_point_jacobi(const TriArgs& T, int64_t t) {
+// A track's point by Jacobi rotations; false if it has none.
+__device__ bool tri_point_jacobi(const TriArgs& T, int64_t t) {
   const uint32_t b = T.track_ptr[t], e = T.track_ptr[t + 1];
-  if (e - b < 2) return;
   double ata[4][4] = {};
   for (uint32_t k = b; k < e; ++k) {
     double a0[4], a1[4];
@@ -263,21 +262,25 @@ __device__ void tri_point_jacobi(const TriArgs& T, int64_t t) {
   double v[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) v[i] = best == 0 ? V[i][0] : best == 1 ? V[i][1] : best == 2 ? V[i][2] : V[i][3];
-  if (fabs(v[3]) < 1e-12) return;  // geometry.rs:139-141
+  if (fabs(v[3]) < 1e-12) return false;  // geometry.rs:139-141
   T.points[3 * t] = v[0] / v[3], T.points[3 * t + 1] = v[1] / v[3], T.points[3 * t + 2] = v[2] / v[3];
-  T.kept[t] = 2;  // triangulated; decided in tri_keep_kernel
+  return true;
 }
 
+// The tracks that tri_point_kernel left.
 __global__ void __launch_bounds__(kTriThreads) tri_rest_kernel(TriArgs T) {
   const uint32_t n = T.rest[T.nt];
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    tri_point_jacobi(T, T.rest[i]);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t t = T.rest[i];
+    if (tri_point_jacobi(T, t)) T.kept[t] = 2;  // triangulated; decided in tri_keep_kernel
+  }
 }
 
-// Every track by Jacobi rotations (a round's problem, see TriRun::run).
-__global__ void __launch_bounds__(kTriThreads) tri_jacobi_kernel(TriArgs T) {
+// The points of a round's problem: every kept track's by Jacobi rotations
+// (see TriRun::run).
+__global__ void __launch_bounds__(kTriThreads) tri_round_kernel(TriArgs T) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < T.nt) tri_point_jacobi(T, t);
+  if (t < T.nt && T.kept[t] == 1) tri_point_jacobi(T, t);
 }
 
 // Reprojection gate (sparse.rs:397-405) and the unit ray of each good
@@ -397,11 +400,15 @@ struct TriRun {
   DevBuf<double> obs_uv, rot, center, intr, points, pn, ray, ctr;
   DevBuf<uint8_t> kept, good;
 
-  // rotations: every point by Jacobi rotations.  A bundle adjustment stops
-  // where the rounding of its start leaves its capped inner solves (centres
-  // 1e-5 of their size apart from starts 1e-12 apart), so a round, whose
-  // triangulation is 1 % of it, keeps the points' last bits; a call for the
-  // points takes the faster and closer inverse iteration.
+  // Which tracks and observations are kept is decided on the inverse
+  // iteration's points for every caller: the two calls keep the same ones, so
+  // that the flags of one name the points of the other's problem, also in
+  // coordinates far from the origin, where the two methods' points differ by
+  // more than rounding (1e-4 m at 20 km).  rotations: the kept points are then
+  // formed again by Jacobi rotations.  A bundle adjustment stops where the
+  // rounding of its start leaves its capped inner solves (centres 1e-5 of
+  // their size apart from starts 1e-12 apart), so a round, whose triangulation
+  // is 1 % of it, keeps the points' last bits.
   void run(const ba_tracks* tr, const double* h_rot, const double* h_center, const double* h_intr,
            double thr, bool rotations, cudaStream_t s) {
     check_tracks(tr);
@@ -441,16 +448,14 @@ struct TriRun {
       check(cudaMemsetAsync(rest.p + nt, 0, 4, s), "memset");
       if (nc > 0) BA_LAUNCH(tri_camera_kernel<<<grid_for(nc, 128), 128, 0, s>>>(T));
       BA_LAUNCH(tri_undistort_kernel<<<grid_for(no, 256), 256, 0, s>>>(T));
-      if (rotations) {
-        BA_LAUNCH(tri_jacobi_kernel<<<grid_for(nt, kTriThreads), kTriThreads, 0, s>>>(T));
-      } else {
-        BA_LAUNCH(tri_point_kernel<<<grid_for(nt, kTriThreads), kTriThreads, 0, s>>>(T));
-        // two or three CTAs on every SM where the tracks are many
-        BA_LAUNCH(
-            tri_rest_kernel<<<std::min(grid_for(nt, kTriThreads), 400u), kTriThreads, 0, s>>>(T));
-      }
+      BA_LAUNCH(tri_point_kernel<<<grid_for(nt, kTriThreads), kTriThreads, 0, s>>>(T));
+      // two or three CTAs on every SM where the tracks are many
+      BA_LAUNCH(
+          tri_rest_kernel<<<std::min(grid_for(nt, kTriThreads), 400u), kTriThreads, 0, s>>>(T));
       BA_LAUNCH(tri_gate_kernel<<<grid_for(no, 256), 256, 0, s>>>(T));
       BA_LAUNCH(tri_keep_kernel<<<grid_for(nt, kTriThreads), kTriThreads, 0, s>>>(T));
+      if (rotations)
+        BA_LAUNCH(tri_round_kernel<<<grid_for(nt, kTriThreads), kTriThreads, 0, s>>>(T));
     }
     uint32_t e = 0;
     check(cudaMemcpyAsync(&e, err.p, 4, cudaMemcpyDeviceToHost, s), "d2h");

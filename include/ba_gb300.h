@@ -354,7 +354,11 @@ ba_status ba_triangulate(const ba_tracks* tracks, const double* rot, const doubl
  * adjustment problem in the context's device memory (sparse.rs:429-449:
  * points of the kept tracks in track order, their kept observations sorted
  * by point; cameras and groups as given; priors optional) without a round
- * trip through the host.  `cams`: rot, center, intr (points ignored).  Then
+ * trip through the host.  The tracks and observations kept are those of
+ * ba_triangulate (its kept and good flags name the problem's points and
+ * observations); the points are formed by another method and may differ from
+ * ba_triangulate's within the accuracy of the normal matrix in 64 bits.
+ * `cams`: rot, center, intr (points ignored).  Then
  * ba_context_solve / ba_context_download as after ba_context_upload.
  * n_points / n_obs receive the problem's sizes.  No counterpart in the
  * reference, which builds the Problem on the host. */
