@@ -496,7 +496,7 @@ struct LmEngine {
   ZSource zsrc{};
   DevBuf<double> camU, camgj, camgs, camX, caml, grpU, grpg, cost_part;
   IterBufs<R> B{};
-  DevBuf<double> lambda, cost, new_cost, rms, sq, sigma;
+  DevBuf<double> lambda, rej_lambda, cost, new_cost, rms, sq, sigma;
   DevBuf<int64_t> n_front, pcg_total;
   DevBuf<int32_t> active, accepted, iters, pcg_iters, any, small, pcg_cap;
   DevBuf<double> log_cost, log_lam;
@@ -738,6 +738,8 @@ struct LmEngine {
     }
     small.alloc(nm, s);
     small.zero();
+    rej_lambda.alloc(nm, s);
+    check(cudaMemsetAsync(rej_lambda.p, 0x7f, 8 * nm, s), "memset");  // 1.4e306: no step yet
     // PCG iteration cap per model: pcg_max_iter, raised to pcg_end_max_iter by
     // the control kernel in the end game; the kernels take the smaller of it
     // and their launch limit (which the autotuner lowers for its trials).
@@ -750,7 +752,7 @@ struct LmEngine {
     }
     const int32_t patience = o.stop_patience > 0 ? o.stop_patience : 1;
     C = Control{lambda, cost, new_cost, rms, sq, n_front, active, accepted, iters, pcg_iters,
-                pcg_total, any, sigma, small, patience, o.max_iter, pcg_cap,
+                pcg_total, any, sigma, small, rej_lambda, patience, o.max_iter, pcg_cap,
                 o.pcg_end_max_iter, o.pcg_end_rel, log_cap, log_cost, log_lam, log_pcg, log_acc};
     if constexpr (sizeof(R) == 4) {
       rec_stale.alloc(nm, s);

@@ -97,6 +97,7 @@ struct Control {
   int32_t* any_active;
   double* sigma;      // per model
   int32_t* small;     // consecutive accepted steps below the 1e-6 decrease
+  double* rej_lambda; // damping of the last rejected step (infinite: none)
   int32_t patience;   // stop after this many (1: the reference's rule)
   int32_t max_iter;
   // End-game PCG cap: once an accepted step decreases a model's cost by less

@@ -42,7 +42,8 @@ class Options:
                                   # cluster_wide: 1024 threads per CTA)
     graph: bool = True            # replay a CUDA graph per LM iteration
     autotune: bool = False        # time PCG configurations on the first solve of a form
-    stop_patience: int = 0        # consecutive small accepted steps before stopping (0/1: ba.rs rule)
+    stop_patience: int = 0        # consecutive small accepted steps before stopping (0/1: ba.rs rule;
+                                  # >= 3: not counting steps that a rejection has damped)
     coarse: bool = False          # mixed form, cluster PCG: two-level preconditioner
     wait_limit_cycles: int = 0    # spin limit of device-side waits (0: ~2 s)
     workspace_limit_bytes: int = 0  # device memory the call may hold (0: no limit) -> BA_OOM

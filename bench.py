@@ -16,7 +16,8 @@ initial state.
 * ``forms``  — FP64 plain form (the reference's block-Jacobi PCG, 400
   iterations), FP32/FP64 mixed form (two-level PCG: block Jacobi plus the
   similarity motions of camera groups, 40 iterations; 60 above 1000 cameras
-  per model; stop after two consecutive small decreases) and, as an
+  per model; stop after two consecutive small decreases, four up to 200
+  cameras) and, as an
   ablation, the mixed form with the reference's block-Jacobi PCG alone (200
   iterations), side by side: final cost of each,
   relative difference from the FP64 form, and the error of every result
@@ -83,9 +84,10 @@ MAX_ITER = 60
 MIXED_PCG_ITERS = 40
 MIXED_PCG_ITERS_LARGE = 60
 MIXED_LARGE_CAMS = 1000
-# The mixed forms stop after two consecutive accepted steps with a relative
-# decrease below 1e-6 (the reference's rule, ba.rs:372-374, stops after one):
-# an FP32 inner solve can give one small decrease before the minimum.
+# The mixed forms stop (above 200 cameras, see below) after two consecutive
+# accepted steps with a relative decrease below 1e-6 (the reference's rule,
+# ba.rs:372-374, stops after one): an FP32 inner solve can give one small
+# decrease before the minimum.
 # Measured with 40 PCG iterations: the 500-camera survey takes one LM
 # iteration more (12 -> 13) and ends 2.1e-6 below the FP64 form; on the
 # 64-model batch 7 models ended up to 1.1e-5 above their FP64 cost with one
@@ -96,11 +98,22 @@ MIXED_STOP_PATIENCE = 2
 # (an inexact-Newton forcing rule: tighter inner solves as the outer iteration
 # converges).  Measured (median of two solves, GB300): without it the 77-camera
 # survey stops 5.5e-6 above its FP64 cost (11.7 ms) and one of the 64 batched
-# models 1.07e-6 above; with it every model of the 77- and 500-camera surveys,
-# the 2000-camera survey and the batch ends at or below its FP64 cost, at
-# 21.4 / 35.2 / 196 / 305 ms against 11.7 / 32.8 / 188 / 273 ms without.
+# models 1.07e-6 above; with it the 500- and the 2000-camera survey end 2e-6
+# below their FP64 cost and every model of the batch within 2e-7 of its own, on
+# every PCG layout that the autotuner can keep.
 MIXED_END_PCG_ITERS = 100
 MIXED_END_REL = 1e-5
+# A small survey's end game depends on rounding, and so on the layout that the
+# autotuner's timing keeps: with the settings above the 77-camera survey ended
+# between 3.9e-6 below and 1.4e-5 above its FP64 cost over 16 layouts, others
+# of 48 and 110 cameras up to 3.9e-5 and 1.2e-5 above.  With a patience of four
+# (which passes over steps that a rejection has damped) and 200 iterations the
+# 77-camera survey ends at least 1.7e-6 below on all of them, the others within
+# 2.3e-6.  At 200 cameras the worst of seven layouts with the settings above is
+# 1.5e-6, at 300 every one is below.
+MIXED_SMALL_CAMS = 200
+MIXED_STOP_PATIENCE_SMALL = 4
+MIXED_END_PCG_ITERS_SMALL = 200
 # Ablation: the mixed form's FP32 records, Schur sums and PCG vectors with the
 # reference's block-Jacobi preconditioner alone, capped at 200 PCG iterations.
 ABLATION_PCG_ITERS = 200
@@ -199,12 +212,18 @@ class ClockSampler:
 # --jtj-recompute: J^T J recomputed in the PCG, no Schur factors stored)
 MIXED_MATRIX_FREE = False
 MIXED_PCG_CAP = MIXED_PCG_ITERS  # set per workload by set_mixed_cap
+STOP_PATIENCE = END_PCG_ITERS = None  # the options', else set by set_mixed_cap
 
 
 def set_mixed_cap(ps):
-    global MIXED_PCG_CAP
-    big = max(p.n_cams for p in ps) > MIXED_LARGE_CAMS
-    MIXED_PCG_CAP = MIXED_PCG_ITERS_LARGE if big else MIXED_PCG_ITERS
+    global MIXED_PCG_CAP, STOP_PATIENCE, END_PCG_ITERS
+    most = max(p.n_cams for p in ps)
+    MIXED_PCG_CAP = MIXED_PCG_ITERS_LARGE if most > MIXED_LARGE_CAMS else MIXED_PCG_ITERS
+    small = most <= MIXED_SMALL_CAMS
+    if STOP_PATIENCE is None:
+        STOP_PATIENCE = MIXED_STOP_PATIENCE_SMALL if small else MIXED_STOP_PATIENCE
+    if END_PCG_ITERS is None:
+        END_PCG_ITERS = MIXED_END_PCG_ITERS_SMALL if small else MIXED_END_PCG_ITERS
 
 
 def form_options(form: str, **kw):
@@ -221,13 +240,13 @@ def form_options(form: str, **kw):
         mf = ("recompute" if MIXED_MATRIX_FREE == "recompute"
               else "matrix_free" if MIXED_MATRIX_FREE else "auto")
         kw.setdefault("coarse", not MIXED_MATRIX_FREE)
-        kw.setdefault("stop_patience", MIXED_STOP_PATIENCE)
-        if MIXED_END_PCG_ITERS > 0:
-            kw.setdefault("pcg_end_max_iter", max(MIXED_END_PCG_ITERS, MIXED_PCG_CAP))
+        kw.setdefault("stop_patience", STOP_PATIENCE)
+        if END_PCG_ITERS > 0:
+            kw.setdefault("pcg_end_max_iter", max(END_PCG_ITERS, MIXED_PCG_CAP))
             kw.setdefault("pcg_end_rel", MIXED_END_REL)
         return Options(precision="mixed", pcg_max_iter=MIXED_PCG_CAP, matrix_free=mf, **kw)
     if form == "mixed_bj":
-        kw.setdefault("stop_patience", MIXED_STOP_PATIENCE)
+        kw.setdefault("stop_patience", STOP_PATIENCE)
         return Options(precision="mixed", pcg_max_iter=ABLATION_PCG_ITERS, coarse=False, **kw)
     return Options(precision="fp64", **kw)
 
@@ -721,7 +740,8 @@ def main():
     ap.add_argument("--mixed-patience", type=int, default=0,
                     help="mixed forms: consecutive small decreases before stopping (0: default)")
     ap.add_argument("--mixed-end-iters", type=int, default=-1,
-                    help="mixed form: end-game PCG cap (-1: default 100, 0: off)")
+                    help="mixed form: end-game PCG cap (-1: default 100, 200 up to 200 cameras; "
+                         "0: off)")
     ap.add_argument("--pcg-kernel", default="auto", choices=["auto", "cluster", "cluster_wide"],
                     help="mixed forms: PCG layout (auto: the autotuner's choice; cluster / "
                          "cluster_wide: one cluster per model of 512- / 1024-thread CTAs)")
@@ -732,16 +752,16 @@ def main():
                     help="points of a single survey (0: the workload's own); a smaller case "
                          "with the same camera network, for profiling")
     args = ap.parse_args()
-    global MIXED_MATRIX_FREE, MIXED_STOP_PATIENCE, MIXED_END_PCG_ITERS, N_POINTS, POINT_KERNEL
+    global MIXED_MATRIX_FREE, STOP_PATIENCE, END_PCG_ITERS, N_POINTS, POINT_KERNEL
     global PCG_KERNEL
     N_POINTS = args.n_points
     POINT_KERNEL = args.point_kernel
     PCG_KERNEL = args.pcg_kernel
     MIXED_MATRIX_FREE = "recompute" if args.jtj_recompute else args.matrix_free
     if args.mixed_patience > 0:
-        MIXED_STOP_PATIENCE = args.mixed_patience
+        STOP_PATIENCE = args.mixed_patience
     if args.mixed_end_iters >= 0:
-        MIXED_END_PCG_ITERS = args.mixed_end_iters
+        END_PCG_ITERS = args.mixed_end_iters
     ws, rank = dist_env()
     if args.stage != "ba":
         out = stage_arm(args, ws, rank)

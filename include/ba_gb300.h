@@ -128,7 +128,11 @@ typedef struct ba_options {
                            the fastest for this and later solves          */
   int32_t stop_patience; /* LM stops after this many consecutive accepted
                            steps with relative decrease < 1e-6; 0 or 1:
-                           the reference's rule (ba.rs:372-374)          */
+                           the reference's rule (ba.rs:372-374); 3 or more:
+                           steps whose damping is still above the last
+                           rejected step's do not count and start the count
+                           over (models of up to about 200 cameras in the
+                           mixed form, whose end game rejects many steps) */
   int32_t coarse;       /* mixed form, cluster PCG: 1 adds a coarse correction
                            to the block-Jacobi preconditioner (the seven
                            similarity motions of each group of consecutive
