@@ -7,9 +7,9 @@
 //    median Sampson error of a pair's matches under the current poses.
 //
 // RANSAC is split into its data-parallel parts.  Hypothesis samples depend
-// on one xorshift stream per pair (each draw depends on the previous), so a
-// thread per pair writes all of its pair's samples first.  Then a thread per
-// hypothesis fits the normalised 8-point F (the null vector of its 8x9
+// on one xorshift stream per pair; a warp draws from 32 places of it at once
+// and writes all of its pair's samples first.  Then a thread per hypothesis
+// fits the normalised 8-point F (the null vector of its 8x9
 // system, rank 2 by removing the smallest singular value); a warp counts a
 // hypothesis' inliers over the pair's correspondences (FP32 with an
 // error bound, FP64 near the threshold: the decisions are the FP64 ones); a

@@ -553,12 +553,11 @@ __host__ __device__ inline uint32_t pcg_blocks(const uint32_t* row_ptr, const Pc
 
 // kAll: shared memory holds every S block of the CTA's rows.
 //
-// Code size: an iteration is one pass over code that each warp runs once, and
-// an FP64 operation takes about seven instruction words here, so straight-
-// line code waits for instruction fetches longer than for its operations.
-// The FP64 form keeps its longest loop rolled (its overhead hides behind the
-// FP64 operations) and shares the exchange and the division as functions:
-// 3.6 µs of a 9.6 µs iteration went into two inlined exchanges before.
+// Code size: an iteration is one pass over code that each warp runs once, so
+// straight-line code waits for its instruction fetches.  The FP64 form keeps
+// its longest loop rolled (its overhead hides behind the FP64 operations) and
+// shares the exchange and the division as functions: 3.6 µs of a 9.6 µs
+// iteration went into two inlined exchanges before.
 //
 // kHalves (FP64, kAll; every row has up to 16 blocks): a block is in lanes l
 // and l + 16, which take three of its rows each: half the operations of the

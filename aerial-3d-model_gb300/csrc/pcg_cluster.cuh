@@ -82,8 +82,14 @@ constexpr uint32_t kCgOwnRow = 0x80000000u;
 constexpr int kCgCache = 12;
 // Rows that a warp takes at once where a row is six lanes' work.
 constexpr int kCgLaneRows = 5;
-// What the choice of kernel counts a slot as.
+// Which models a cluster serves (LmEngine::try_cluster) is a rule of their own
+// sizes, not of what this kernel happens to need: 24 floats a neighbour slot, 4
+// bytes a block's slot and a static part of 1616 + threads / 2 bytes beside the
+// row state.  The kernel gets by with less, so that every model it serves fits;
+// but with the kernel a model would change the layout of its sums, and the
+// mixed form's end game, which depends on their rounding, its result.
 constexpr int kCgCacheAsk = 24;
+constexpr size_t cg_static_ask(int threads) { return 1616 + (size_t)threads / 2; }
 
 struct CgJob {
   int32_t model;
@@ -176,7 +182,7 @@ __device__ __forceinline__ bool cg_bulk_wait(uint64_t* bar, long long spin) {
 }
 
 // A block's cache slot as kept in shared memory: the CTA's own row in the low
-// 15 bits under bit 15, else the slot (a slot takes 96 bytes and a row 320 of
+// 15 bits under bit 15, else the slot (a slot takes 48 bytes and a row 320 of
 // the same shared memory, so both numbers stay far below 2^15).
 constexpr uint32_t kCgOwnSlot = 0x8000u;
 __device__ __forceinline__ uint32_t cg_slot16(uint32_t e) {
@@ -549,7 +555,7 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
   const uint32_t* subs = A.cap_subs > 0 ? sSub : A.sub_ent + sub0;
 #define CGROW(lr) (rs + (size_t)(lr) * kCgPitch)
   // x = 0, r = b, z = M r, p(prev) = 0 (ba.rs:164-168).  Inner products:
-  // each lane accumulates its component's FP64 products over the warp's rows;
+  // each lane accumulates its component's FP32 products over the warp's rows;
   // the lanes are summed once per phase.
   float drz = 0.0f, dbb = 0.0f;
   for (uint32_t lr = warp; lr < nrows; lr += kCgWarps) {

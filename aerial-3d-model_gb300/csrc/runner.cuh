@@ -1021,10 +1021,8 @@ struct LmEngine {
     const detail::CgKernel kfn = detail::cg_kernel(coarse, threads, false);
     cudaFuncAttributes fa{};
     check(cudaFuncGetAttributes(&fa, kfn), "func attr");
-    // (the static arrays are counted as no less than when the choices below
-    // were measured)
     const size_t avail =
-        (size_t)smem_optin - std::max(fa.sharedSizeBytes, (size_t)(1616 + threads / 2));
+        (size_t)smem_optin - std::max(fa.sharedSizeBytes, cg_static_ask(threads));
     // Row state takes at most half of the shared memory (the rest caches S
     // blocks); with the coarse correction, which needs far fewer PCG
     // iterations, rows may take all of it and S is read from L2.
@@ -1070,8 +1068,8 @@ struct LmEngine {
     const size_t cache_bytes = (size_t)kp.cap * kCgCacheAsk * 4;
     if (row_bytes + coarse_bytes + cache_bytes >= avail)
       return unusable("row state and neighbour cache do not fit");
-    // Whether the clusters serve: with every S block cached that fits beside a
-    // slot of 4 bytes each.
+    // Whether the clusters serve, by the rule at kCgCacheAsk: with every S block
+    // cached that fits beside a slot of 4 bytes each.
     const size_t ask_bytes = row_bytes + coarse_bytes + cache_bytes;
     size_t smem = ask_bytes +
                   std::min<size_t>(cp.max_blocks, (avail - ask_bytes) / (36 * 4 + 4)) * (36 * 4 + 4);

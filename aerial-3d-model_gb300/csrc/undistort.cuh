@@ -31,10 +31,13 @@ __device__ __forceinline__ double reciprocal_near(double d) {
 }
 
 // x / d with r = 1 / d to 2^-45 or better: q = x r and one residual
-// correction, which rounds x / d + (x / d - q)(1 - d r), i.e. the quotient but
-// for 2^-36 of a last place (Markstein, IBM J. Res. Dev. 34, 1990).  The
-// residual is exact where neither it nor q leaves the normal range; outside
-// of 2^-900 .. 2^900 (and for zero, infinite or NaN values) the division.
+// correction (Markstein, IBM J. Res. Dev. 34, 1990).  q is off by up to 2^8
+// last places, so the residual x - q d has some 60 bits and is rounded to 53:
+// an error of 2^-45 of a last place of q; r adds 2^8 times 2^-45 of one.  The
+// result is x / d rounded but for 2^-36 of a last place (with r rounded to
+// nearest q is off by one and the residual exact).  For q or r outside of
+// 2^-900 .. 2^900 (and zero, infinite or NaN values) the division; an x below
+// 2^-960, whose residual would be subnormal, is divided to its own spacing.
 __device__ __forceinline__ double quotient_by(double x, double d, double r) {
   const double q = mul_any(x, r);
   const uint32_t eq = ((uint32_t)__double2hiint(q) >> 20) & 0x7ffu;
