@@ -223,7 +223,10 @@ struct SummaryRun {
       const bool in_smem = nc <= kSmemHistCams;
       const size_t smem = kDepthKeys * 8 + (in_smem ? (size_t)nc * 4 : 0);
       auto kernel = in_smem ? camera_summary_kernel<true> : camera_summary_kernel<false>;
-      check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+      // The limit belongs to the process: the same value from every call, so that
+      // none lowers it between another thread's setting and its launch.
+      check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(kDepthKeys * 8 + (in_smem ? kSmemHistCams * 4 : 0))),
             "summary smem");
       int occ = 0;
       check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kNbThreads, smem),
