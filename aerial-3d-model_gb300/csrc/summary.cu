@@ -78,14 +78,19 @@ struct CamArgs {
   double agl;
   int max_nb;
   uint32_t* hist_global;  // gridDim.x * nc counts when not in shared memory
-  uint64_t* key_global;   // [n_obs] depth keys of cameras beyond kDepthKeys
+  uint32_t keys;          // depth keys of a camera in shared memory
+  uint64_t* key_global;   // [n_obs] depth keys of cameras beyond `keys`
   uint32_t* nb;           // [nc * max_nb], UINT32_MAX padded
   uint32_t* shared;       // [nc * max_nb], 0 padded
   int32_t* n_nb;          // [nc]
   double* range;          // [nc * 2]
 };
 
-constexpr uint32_t kDepthKeys = 8192;  // depth keys of a camera in shared memory
+// Depth keys of a camera in shared memory: where they and the counts leave room
+// for one CTA an SM only (above some 12,000 cameras), the fewer (13,000 cameras
+// of 60 observations: 1.91 -> 1.42 ms, of 2000: 10.2 -> 8.9 although their keys
+// are then in global memory; 24,576 of 30: 3.79 -> 3.18).
+constexpr uint32_t kDepthKeys = 8192, kDepthKeysFew = 1024;
 
 // Camera-frame depth of a point, (R (X - C)).z with the products summed left
 // to right and no fused multiply-add (Pose::to_cam, geometry.rs:57-59, as
@@ -113,13 +118,13 @@ __global__ void __launch_bounds__(kNbThreads) camera_summary_kernel(CamArgs A) {
   __shared__ uint64_t red[kNbThreads / 32 + 1];
   __shared__ uint32_t bytes[256], found[3];
   uint64_t* skey = reinterpret_cast<uint64_t*>(smem_raw);
-  uint32_t* hist = kSmem ? reinterpret_cast<uint32_t*>(skey + kDepthKeys)
+  uint32_t* hist = kSmem ? reinterpret_cast<uint32_t*>(skey + A.keys)
                          : A.hist_global + (size_t)blockIdx.x * A.nc;
   for (int64_t c = threadIdx.x; c < A.nc; c += kNbThreads) hist[c] = 0;
   __syncthreads();
   for (int64_t a = blockIdx.x; a < A.nc; a += gridDim.x) {
     const uint32_t b = A.cam_ptr[a], n = A.cam_ptr[a + 1] - b;
-    uint64_t* key = n <= kDepthKeys ? skey : A.key_global + b;
+    uint64_t* key = n <= A.keys ? skey : A.key_global + b;
     const double R[3] = {A.rot[9 * a + 6], A.rot[9 * a + 7], A.rot[9 * a + 8]};
     const double C[3] = {A.center[3 * a], A.center[3 * a + 1], A.center[3 * a + 2]};
     for (uint32_t i = threadIdx.x; i < n; i += kNbThreads) {
@@ -221,7 +226,8 @@ struct SummaryRun {
     }
     if (nc > 0) {
       const bool in_smem = nc <= kSmemHistCams;
-      const size_t smem = kDepthKeys * 8 + (in_smem ? (size_t)nc * 4 : 0);
+      uint32_t keys = kDepthKeys;
+      size_t smem = keys * 8 + (in_smem ? (size_t)nc * 4 : 0);
       auto kernel = in_smem ? camera_summary_kernel<true> : camera_summary_kernel<false>;
       // The limit belongs to the process: the same value from every call, so that
       // none lowers it between another thread's setting and its launch.
@@ -231,12 +237,17 @@ struct SummaryRun {
       int occ = 0;
       check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kNbThreads, smem),
             "occupancy");
+      if (occ < 2) {
+        keys = kDepthKeysFew, smem -= (kDepthKeys - kDepthKeysFew) * 8;
+        check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kNbThreads, smem),
+              "occupancy");
+      }
       const unsigned grid =
           (unsigned)std::min<int64_t>(nc, (int64_t)std::max(occ, 1) * std::max(n_sm, 1));
       if (!in_smem) A(hist, (int64_t)grid * nc);
-      DevBuf<uint64_t> key(no > (int64_t)kDepthKeys ? no : 1, s);
+      DevBuf<uint64_t> key(no > (int64_t)keys ? no : 1, s);
       CamArgs ca{nc,     cam_ptr, cam_obs, pt_ptr, obs_cam, obs_pt, rot,  center, points,
-                 agl,    max_nb,  hist,    key,    nb,      shared, n_nb, range};
+                 agl,    max_nb,  hist,    keys,   key,     nb,     shared, n_nb, range};
       BA_LAUNCH(kernel<<<grid, kNbThreads, smem, s>>>(ca));
     }
     if (np > 0) BA_LAUNCH(points_f32_kernel<<<grid_for(3 * np, 256), 256, 0, s>>>(3 * np, points, pts32));
