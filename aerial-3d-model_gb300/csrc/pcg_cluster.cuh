@@ -271,17 +271,45 @@ struct CgInbox {
   }
 };
 
+// The totals of an inbox, in every thread.  Of
+// 512 threads every warp sums the inbox: that saves the CTA barrier after it,
+// and the 16 warps fetch the same instructions at the same time.  32 warps
+// issue their sums for longer than the barrier takes: there warp 0 sums for
+// all, and lane 0 runs post(v) before that barrier (77 cameras, four steps of
+// 400 iterations without the coarse correction: every warp 11.95 ms, warp 0
+// 10.6; 250 cameras 16.3 and 14.9).
+template <int kThreads, int N, typename Post>
+__device__ __forceinline__ void cg_totals(const DFloat (*inbox)[4], int csize, int lane,
+                                          DFloat* tot, DFloat (&v)[N], Post&& post) {
+  if constexpr (kThreads == kCgThreads) {
+    const CgInbox<N> in(inbox, csize, lane);
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = in.total(i);
+  } else {
+    if (threadIdx.x < 32) {
+      const CgInbox<N> in(inbox, csize, lane);
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        v[i] = in.total(i);
+        if (lane == 0) tot[i] = v[i];
+      }
+      if (lane == 0) post(v);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = tot[i];
+  }
+}
+
 // Inner products: a warp sums its rows' products in FP32 (a few rows of six
 // components); the warps' partials are summed as double-floats over the CTA
 // by warp 0, which pushes them to every CTA of the cluster, and after the
-// cluster barrier every warp sums its CTA's inbox (CgInbox): the same partials
+// cluster barrier the CTA's inbox is summed (cg_totals): the same partials
 // in the same order everywhere, so every thread of the cluster holds
 // bit-identical totals.  wv: N (<= 4) values held by lane 0 of every warp.
 // While warp 0 sums and pushes, warps 1.. run side(w) with w = warp - 1 (the
 // coarse group sums, which read the same row state after the same CTA
-// barrier).  That every warp sums the inbox, not warp 0 for the others, saves
-// the CTA barrier after it, and the 16 warps fetch the same instructions at
-// the same time.
+// barrier).
 //
 // Exchange by push: before the cluster barrier, lane r of warp 0 stores the
 // CTA's partials into CTA r's inbox (inbox[source rank][value]); after it,
@@ -426,6 +454,7 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
   constexpr int kCgWarps = kThreads / 32;
   __shared__ float wsm[kCgWarps * 4];
   __shared__ DFloat inbox[3][kCgMaxCluster][4];  // reduction inboxes (push)
+  __shared__ DFloat tot[4];    // an exchange's totals (1024 threads)
   __shared__ float lens_p[4];  // the lens row's p, pushed by its owner
   __shared__ uint64_t stage_bar;  // completion of the S blocks' bulk copy
   extern __shared__ __align__(16) unsigned char cg_smem[];
@@ -584,8 +613,9 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
       cg_group_sums_push<kCgWarps - 1>(cl, w, ngr, sGrp, goff, sW, rs, kCgR, wall_r);
   });
   {
-    const CgInbox<2> in(inbox[1], (int)csz, lane);
-    rz = in.total(0).hi, b2 = in.total(1).hi;
+    DFloat v[2];
+    cg_totals<kThreads>(inbox[1], (int)csz, lane, tot, v, [](auto&) {});
+    rz = v[0].hi, b2 = v[1].hi;
   }
   if constexpr (kCoarse) {
     for (int o = warp - 1; o >= 0 && o < nco; o += kCgWarps - 1)
@@ -609,7 +639,9 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
     }
     const float w1[1] = {cg_sum8f(drz0)};
     cg_exchange<kCgWarps, 1>(cl, w1, wsm, inbox[2], [](int) {});
-    rz = CgInbox<1>(inbox[2], (int)csz, lane).total(0).hi;
+    DFloat v[1];
+    cg_totals<kThreads>(inbox[2], (int)csz, lane, tot, v, [](auto&) {});
+    rz = v[0].hi;
   } else {
     for (uint32_t lr = warp; lr < nrows; lr += kCgWarps) {
       const float* st = CGROW(lr);
@@ -622,8 +654,10 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
   for (int32_t it = 0; it < max_it; ++it) {
     const int cur = it & 1, prv = cur ^ 1;
     // p = z + β p of every cached row, once: the rows' owners push z only.
-    for (uint32_t t = threadIdx.x; t < A.cap_cache * 6; t += kThreads) cp[t] = cz[t] + cp[t] * bf;
-    __syncthreads();
+    if (A.cap_cache > 0) {
+      for (uint32_t t = threadIdx.x; t < A.cap_cache * 6; t += kThreads) cp[t] = cz[t] + cp[t] * bf;
+      __syncthreads();
+    }
     // q = S p: a lane per block of a row.
     for (uint32_t lr = warp; lr < nrows; lr += kCgWarps) {
       float* st = CGROW(lr);
@@ -700,6 +734,9 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
       }
 #pragma unroll
       for (int g = 0; g < kCgLaneRows; ++g) {
+        // (uniform; 512 threads have three or four rows a warp, and the test
+        // there takes longer than it saves)
+        if (kThreads == kCgThreadsWide && l0 + g * kCgWarps >= nrows) break;
         const float pg = __shfl_sync(kFull, pi, 6 * g + ci), qg = __shfl_sync(kFull, qi, 6 * g + ci);
         const float vg = __shfl_sync(kFull, v, 6 * g + ci);
         const int32_t lg = __shfl_sync(kFull, lp, 6 * g);
@@ -722,21 +759,34 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
     float af;
     bool stop;
     {
-      const CgInbox<4> in(inbox[0], (int)csz, lane);
-      DFloat pq = in.total(0);
-      if (lens >= 0) {
-        // The lens row's q gets the transposed camera terms; its share of
-        // p.q is p_g . (sum S_cg^T p_c), with p_g pushed by its owner before
-        // the barrier.
+      // The lens row's q gets the transposed camera terms; its share of p.q is
+      // p_g . (sum S_cg^T p_c), with p_g pushed by its owner before the barrier.
+      DFloat pq;
+      auto lens_q = [&](int c, DFloat t) {
+        float* q = CGROW((uint32_t)lens - J.row0) + kCgQ;
+        q[c] = df_sum(DFloat{q[c], 0.0f}, t).hi;
+      };
+      if constexpr (kThreads == kCgThreads) {
+        const CgInbox<4> in(inbox[0], (int)csz, lane);
+        pq = in.total(0);
+        if (lens >= 0) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const DFloat t = in.total(1 + c);
-          pq = df_sum(pq, df_scale(lens_p[c], t));
-          if (lens_here && threadIdx.x == 0) {
-            float* q = CGROW((uint32_t)lens - J.row0) + kCgQ;
-            q[c] = df_sum(DFloat{q[c], 0.0f}, t).hi;
+          for (int c = 0; c < 3; ++c) {
+            const DFloat t = in.total(1 + c);
+            pq = df_sum(pq, df_scale(lens_p[c], t));
+            if (lens_here && threadIdx.x == 0) lens_q(c, t);
           }
         }
+      } else {
+        DFloat v[4];
+        cg_totals<kThreads>(inbox[0], (int)csz, lane, tot, v, [&](auto& t) {
+          if (lens_here)
+            for (int c = 0; c < 3; ++c) lens_q(c, t[1 + c]);
+        });
+        pq = v[0];
+        if (lens >= 0)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) pq = df_sum(pq, df_scale(lens_p[c], v[1 + c]));
       }
       // ba.rs:174 breaks on a vanishing p.q; an FP32 quotient needs it normal
       stop = fabsf(pq.hi) < 1.17549435e-38f;
@@ -747,7 +797,8 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
         cg_coarse_dot(sEi, A.cap_dim, cD, o, wr_cur, wall_q, af, scf);
     ++spmv;
     if (stop) break;
-    if (kCoarse || lens_here) __syncthreads();  // c and the lens row's q
+    // c, and the lens row's q
+    if (kCoarse || (kThreads == kCgThreads && lens_here)) __syncthreads();
     float drr = 0.0f, drz2 = 0.0f;
     for (uint32_t l0 = warp; l0 < nrows; l0 += kCgLaneRows * kCgWarps) {
       const uint32_t lr = l0 + gi * kCgWarps;
@@ -770,6 +821,7 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
       }
 #pragma unroll
       for (int g = 0; g < kCgLaneRows; ++g) {
+        if (kThreads == kCgThreadsWide && l0 + g * kCgWarps >= nrows) break;
         const float rg = __shfl_sync(kFull, ri, 6 * g + ci), zg = __shfl_sync(kFull, zi, 6 * g + ci);
         if (vl && l0 + g * kCgWarps < nrows) {
           drr += rg * rg;
@@ -786,8 +838,9 @@ static __global__ void __launch_bounds__(kThreads, kCtas) pcg_cluster_kernel(CgA
                                          wall_r + (size_t)prv * A.cap_dim);
     });
     {
-      const CgInbox<2> in(inbox[1], (int)csz, lane);
-      const float rr = in.total(0).hi, rz1 = in.total(1).hi;
+      DFloat v[2];
+      cg_totals<kThreads>(inbox[1], (int)csz, lane, tot, v, [](auto&) {});
+      const float rr = v[0].hi, rz1 = v[1].hi;
       bf = rz1 / rz;  // ba.rs:189-190
       rz = rz1;
       if (rr < (float)A.tol * b2) break;  // ba.rs:182
