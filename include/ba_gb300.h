@@ -360,8 +360,8 @@ ba_status ba_triangulate(const ba_tracks* tracks, const double* rot, const doubl
  * by point; cameras and groups as given; priors optional) without a round
  * trip through the host.  The tracks and observations kept are those of
  * ba_triangulate (its kept and good flags name the problem's points and
- * observations); the points are formed by another method and may differ from
- * ba_triangulate's within the accuracy of the normal matrix in 64 bits.
+ * observations); the points may differ from ba_triangulate's in their last
+ * digits (by less than 2^-26 of their distance to a camera).
  * `cams`: rot, center, intr (points ignored).  Then
  * ba_context_solve / ba_context_download as after ba_context_upload.
  * n_points / n_obs receive the problem's sizes.  No counterpart in the

@@ -4,10 +4,11 @@ decisions are close (a gate in the middle of the residuals, rays near the
 smallest angle, mismatches, one camera twice) and in coordinates far from the
 origin, where rounding moves a point by more than its last digits.
 
-The points are formed by another method; both are eigenvectors of the same
+The points may be formed by another method; both are eigenvectors of the same
 normal matrix in 64 bits, so they differ by its sensitivity at most: a matrix
 rounded in its last place moves the eigenvector by eps |A| / gap, of which each
-side makes a few (8 a side are allowed)."""
+side makes a few (8 a side are allowed).  And they differ by no more than the
+header says, 2^-26 of the distance to a camera."""
 import numpy as np
 import pytest
 
@@ -71,3 +72,5 @@ def test_a_round_keeps_what_triangulation_keeps(offset, thr):
     # the unit eigenvector's move, and that of its last component (1 / size)
     move = 16 * 2.0**-52 * w[:, 3] / (w[:, 1] - w[:, 0]) * size
     assert (np.linalg.norm(a - b, axis=1) / size <= move + 2.0**-50).all()
+    dist = np.linalg.norm(a - C[cam[ptr[:-1][kept]]], axis=1)
+    assert (np.linalg.norm(a - b, axis=1) <= 2.0**-26 * dist).all()
