@@ -93,7 +93,8 @@ struct PcgArgs {
   const R* pre;  // block-Jacobi inverses, computed in FP64, stored in R
   const R* b;
   R* x;
-  R* pblk;  // [nz][6] p(prev) of blocks that shared memory does not hold
+  R* pblk;  // [nz][6] p(prev) of blocks that shared memory does not hold (no memory of
+            // its own: the sub-segments' sums, dead between assembly and the next Schur pass)
   const int32_t* lens_row;  // [nm]: the model's single lens block row, or -1
   const int32_t* lens_pos;  // [nb]: block index of (row, lens row), or -1
   const uint32_t* diag_pos; // [nb]: block index of the diagonal block

@@ -509,11 +509,9 @@ struct LmEngine {
   DevBuf<int32_t> cta_job0;
   DevBuf<unsigned long long> bar, bar_base;  // matrix-free kernel
   DevBuf<double> pcg_part;
-  // Grid kernel: sequence numbers, exchange words (partial sums, z) and the
-  // previous p of blocks that shared memory does not hold.
+  // Grid kernel: sequence numbers, exchange words (partial sums, z).
   DevBuf<unsigned long long> pcg_epoch;
   DevBuf<PcgWord> pcg_words, pcg_said, pcg_zx;
-  DevBuf<R> pblk;
   DevBuf<int32_t> lens_row, lens_pos;
   uint32_t smem_rows = 0, smem_blocks = 0;
   uint32_t sub_len = kSubLen;  // Schur pairs per warp sub-segment
@@ -960,12 +958,15 @@ struct LmEngine {
     // Sequence numbers start at 0 in every word; a launch's first is 1.
     pcg_epoch.alloc(ctx.nm, s), pcg_words.alloc(3 * kPartPitch * (size_t)plan.ncta, s);
     pcg_zx.alloc(detail::at_least_1(ctx.nb) * kZRowWords, s);
-    pcg_said.alloc(3 * kSaidPitch * (size_t)ctx.nm, s);
+    bool led = false;
+    for (const PcgJob& j : plan.jobs) led = led || j.gsize > kDirectCtas;
+    pcg_said.alloc(led ? 3 * kSaidPitch * (size_t)ctx.nm : 1, s);
     pcg_epoch.zero(), pcg_words.zero(), pcg_said.zero(), pcg_zx.zero();
     uint32_t most = 0;
     for (const PcgJob& j : plan.jobs)
       most = std::max(most, pcg_blocks(SB.h_row_ptr.data(), j, h_lens[j.model]));
-    pblk.alloc(most > smem_blocks ? (size_t)SB.nz * 6 : 1, s);
+    if (most > smem_blocks && 2 * SB.nsub < SB.nz)  // (a block has a sub-segment at least)
+      throw std::runtime_error("PCG plan: blocks without sub-segments");
     // The form for short rows: all blocks in shared memory, and 16 a row or
     // fewer (the lens row multiplies one).
     pcg_fn = (void*)pcg_kernel<R>;
@@ -987,7 +988,7 @@ struct LmEngine {
     }
     check(cudaStreamSynchronize(s), "sync");  // host plan vectors
     pa = PcgArgs<R>{jobs, cta_job0, pcg_epoch, pcg_words, pcg_said, pcg_zx, plan.ncta, SB.row_ptr,
-                    SB.col_idx, S, pre, g, x, pblk, lens_row, lens_pos, SB.diag_pos, smem_rows,
+                    SB.col_idx, S, pre, g, x, nullptr, lens_row, lens_pos, SB.diag_pos, smem_rows,
                     smem_blocks, active, pcg_iters, pcg_limit, o.pcg_tol, ctx.err,
                     o.wait_limit, o.hold_cta};
     pa.cap = pcg_cap;
@@ -1485,6 +1486,8 @@ struct LmEngine {
       check(cudaLaunchKernelEx(&cfg, detail::cg_kernel(use_coarse, cl_threads, cl_two), ca),
             "pcg cluster launch");
     } else {
+      // likewise the previous p of blocks that shared memory does not hold
+      pa.pblk = (R*)part.p;
       void* args[] = {&pa};
       check(cudaLaunchCooperativeKernel(pcg_fn, dim3(plan.ncta), dim3(kPcgThreads),
                                         args, smem_bytes, s),
