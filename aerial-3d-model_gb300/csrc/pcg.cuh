@@ -65,7 +65,10 @@ struct __align__(16) PcgWord {
 // exchange): partials side by side 1710 / 2790 / 6570, 64 bytes apart
 // 1770 / 1810 / 2290; pushed into an inbox per reader 2260 / 2660 / 4170.
 constexpr int kPartPitch = 4;
-constexpr int kZRowWords = 8;
+// (a row's z: 96 of 128 bytes in FP64, 32 of 64 in FP32, whose rows 128 bytes
+// apart took the same time: 250 cameras 21.7 ms, now 21.0)
+template <typename R>
+constexpr int kZRowWords = sizeof(R) == 8 ? 8 : 4;
 constexpr int kSaidPitch = 8;
 
 // Groups of up to this many CTAs: every CTA collects every partial and forms
@@ -85,7 +88,7 @@ struct PcgArgs {
   unsigned long long* epoch;  // [nm] last sequence number of each model's earlier launches
   PcgWord* part;              // [3][ncta][kPartPitch] partial sums of the three exchanges
   PcgWord* said;              // [nm][3][kSaidPitch] the leader's result of each exchange
-  PcgWord* zx;                // [nb][kZRowWords] z = M r, gathered by neighbours
+  PcgWord* zx;                // [nb][kZRowWords<R>] z = M r, gathered by neighbours
   int32_t ncta;
   const uint32_t* row_ptr;
   const uint32_t* col_idx;
@@ -647,7 +650,7 @@ __device__ bool pcg_job(const PcgArgs<R>& A, const PcgJob& J, double* wsm, doubl
       for (int j = 0; j < 6; ++j) z[j] = st[12 + j];
       return;
     }
-    const PcgWord* w = A.zx + (size_t)col * kZRowWords;
+    const PcgWord* w = A.zx + (size_t)col * kZRowWords<R>;
     if (zx_load(w, tag, z)) return;
     const long long t0 = clock64();
     int tries = 0;
@@ -683,7 +686,7 @@ __device__ bool pcg_job(const PcgArgs<R>& A, const PcgJob& J, double* wsm, doubl
       zi += st[30 + 6 * ci + j] * rj;
     }
     double a = 0.0, bb = 0.0;
-    zx_store(A.zx + (size_t)row * kZRowWords, base + 2, zi, lane);
+    zx_store(A.zx + (size_t)row * kZRowWords<R>, base + 2, zi, lane);
     if (vl) {
       st[ci] = (R)0;
       st[6 + ci] = ri;
@@ -888,7 +891,7 @@ __device__ bool pcg_job(const PcgArgs<R>& A, const PcgJob& J, double* wsm, doubl
         const R rj = __shfl_sync(kFull, ri, j);
         zi += st[30 + 6 * c + j] * rj;
       }
-      zx_store(A.zx + (size_t)row * kZRowWords, tag + 2, zi, lane);
+      zx_store(A.zx + (size_t)row * kZRowWords<R>, tag + 2, zi, lane);
       if (vl) {
         st[6 + ci] = ri;
         st[12 + ci] = zi;

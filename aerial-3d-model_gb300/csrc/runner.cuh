@@ -957,7 +957,7 @@ struct LmEngine {
     detail::h2d(cta_job0, plan.cta_job0, s);
     // Sequence numbers start at 0 in every word; a launch's first is 1.
     pcg_epoch.alloc(ctx.nm, s), pcg_words.alloc(3 * kPartPitch * (size_t)plan.ncta, s);
-    pcg_zx.alloc(detail::at_least_1(ctx.nb) * kZRowWords, s);
+    pcg_zx.alloc(detail::at_least_1(ctx.nb) * kZRowWords<R>, s);
     bool led = false;
     for (const PcgJob& j : plan.jobs) led = led || j.gsize > kDirectCtas;
     pcg_said.alloc(led ? 3 * kSaidPitch * (size_t)ctx.nm : 1, s);
