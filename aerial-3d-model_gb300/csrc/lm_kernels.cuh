@@ -1856,10 +1856,11 @@ static __global__ void control_kernel(int64_t nm, Control C) {
     // An end game of inexact steps rejects many, and a step with the damping
     // that a rejection raised is small whatever is left to gain: a patience of
     // three or more counts steps that are back at the rejected one's damping.
-    // (77 cameras, rounding of 16 layouts: a patience of two ended -3.9e-6 ..
-    // 1.4e-5 of the FP64 cost on one survey, 3e-6 .. 1.6e-5 at worst on three
-    // others; of four, with 200 PCG iterations in the end game, up to 8.6e-6
-    // counting damped steps and 2.3e-6 without.)  A patience of two keeps its
+    // (Nine surveys of 48 to 200 cameras on 16 layouts: with a patience of two
+    // 38 of 144 solves end more than 1e-6 above the FP64 cost, up to 3.9e-5; of
+    // four, with 200 PCG iterations in the end game, 4, up to 2.8e-6.  Counting
+    // damped steps that setting left surveys of 77 and 48 cameras up to 5.2e-6
+    // and 5.4e-6 above where it ends below.)  A patience of two keeps its
     // count, and solves with it their results.
     if (C.patience >= 3 && lam > C.rej_lambda[m]) {
       C.small[m] = 0;

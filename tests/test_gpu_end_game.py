@@ -4,8 +4,9 @@ of up to 200 cameras; the rounding is varied by the order of the points (the
 order of every sum over them) and the PCG kernel (threads per CTA, autotuned
 layouts).
 
-Bound: the FP64 form's cost depends on the order of its sums by 1.17e-5 (the
-reference's stop rule, four permuted orders of a 500-camera survey); the mixed
+Bound: the cost at which the reference's stop rule ends an FP64 solve depends
+on the order of its sums by 1.17e-5 (four orders of a 500-camera survey on the
+CPU; these small surveys on the GPU: 2e-8); the mixed
 form, which stops after four undamped steps below 1e-6 each, has to end less
 than half of that above it.  The stop itself is checked on the iteration log."""
 import numpy as np
@@ -23,7 +24,8 @@ def reordered(p, seed):
     o = np.argsort(to[p.obs_pt], kind="stable")
     pts = np.empty_like(p.points)
     pts[to] = p.points
-    return Problem(intr=p.intr, rot=p.rot, center=p.center, cam_group=p.cam_group, points=pts,
+    return Problem(intr=p.intr.copy(), rot=p.rot.copy(), center=p.center.copy(),
+                   cam_group=p.cam_group, points=pts,
                    obs_cam=np.ascontiguousarray(p.obs_cam[o]),
                    obs_pt=np.ascontiguousarray(to[p.obs_pt][o]),
                    obs_uv=np.ascontiguousarray(p.obs_uv[o]), prior_mask=p.prior_mask,
